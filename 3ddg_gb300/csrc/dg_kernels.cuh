@@ -1,10 +1,12 @@
 // sm_103a kernels for one stage of the DG right-hand side and its RK update.
 //
 // Two launches per RK stage (one without diffusion):
-//   ldg_gradient_kernel  G_a = -D_c d(drho)/dx_a by LDG with the central flux
+//   ldg_gradient_kernel (FP32), ldg_gradient_fix_kernel (FP64, fix_kernels.cuh)
+//                        G_a = -D_c d(drho)/dx_a by LDG with the central flux
 //                        (Element::OperateQFromDRho, cppsrc/Element.cpp:623-690;
 //                        stored pre-multiplied by -D_c, the diffusive flux)
-//   stage_kernel (FP64), incr_stage_kernel (FP32 increment form)
+//   stage_fix_kernel (FP64, fix_kernels.cuh), incr_stage_kernel (FP32
+//                        increment form)
 //                        volume + face terms of the advection operator
 //                        (Element::OperateUFromV, cppsrc/Element.cpp:475-620),
 //                        LDG divergence (Element::OperateDRhoFromQ, :691-758),
@@ -21,19 +23,18 @@
 //     x = (1/w) D f - (1/(q w)) (M^-1 e_0 F_0 + M^-1 e_N F_N),  D = M^-1 S,
 // with D and the lift columns computed once on the host in FP64.
 //
-// FP64 (bound by the FP64 pipe): every constant factor is folded on the host
-// into the per-launch operator (OpConst): the RK stage weight ca, 1/w_a and
-// the equations' lift scales go into per-axis copies of D and into the
-// face-flux coefficients, the gradient carries -D_c so that the LDG
-// divergence and the mass-flux divergence share one line sum, and the sponge
-// folds into the RK combination (its per-element weight tabulated by the
-// host).  The element's face nodes are dealt out densely to its threads so
-// that no warp issues face arithmetic for lanes that have none; each stage
-// writes the volume fluxes of its output for the next stage to read (flux
-// modes), so no face neighbour's flux is evaluated twice; and at K = 5 the
-// line sums use the even-odd split of the centro-antisymmetric D (LineEO),
-// with line owners packed densely two elements per CTA, instead of per-node
-// sums of 2 (K + 2) FMAs per axis.
+// FP64: every constant factor is folded on the host into the per-launch
+// operator (OpConst): the RK stage weight ca, 1/w_a and the equations' lift
+// scales go into per-axis copies of D and into the face-flux coefficients, the
+// gradient carries -D_c so that the LDG divergence and the mass-flux
+// divergence share one line sum, and the sponge folds into the RK combination
+// (its per-element weight tabulated by the host).  The kernels of
+// fix_kernels.cuh evaluate the folded line operators in block fixed point;
+// ldg_gradient_kernel and stage_kernel below sum every node's three lines in
+// FP64, for operators that have no such form (matrix files whose D is not
+// centro-antisymmetric).  Each stage writes the volume fluxes of its output
+// for the next stage to read (flux modes), so no face neighbour's flux is
+// evaluated twice.
 //
 // FP32 (bound by the L1 data pipe, load latency and issue): for K >= 5 line
 // owners (a warp per axis, a lane per line) evaluate their line's two face
@@ -347,74 +348,6 @@ __device__ __forceinline__ int line_base(int t)
     return A == 0 ? t : (A == 1 ? (t % K) * K * K + t / K : t * K);
 }
 
-// Even-odd form of one axis's line operator (FP64 line owners).  D is
-// centro-antisymmetric, D[K-1-i][K-1-j] = -D[i][j], and the lift columns are
-// mirrored, L0[K-1-i] = SIG LN[i]; with e_j = v_j + v_{K-1-j},
-// o_j = v_j - v_{K-1-j} (j < H = K/2), s = f0 + fN, d = f0 - fN:
-//   P_i = sum_j E[i][j] e_j + Dc[i] v_H,  Q_i = sum_j O[i][j] o_j,
-//   out_i = P_i + Q_i,  out_{K-1-i} = Q_i - P_i   (i < H; the lift terms
-//   A s, B d are added to P or Q by SIG),
-//   out_H = sum_j Dm[j] o_j + Lm (s or d)   (K odd),
-// E = (D[i][j] + D[i][K-1-j]) / 2, O = (D[i][j] - D[i][K-1-j]) / 2,
-// A = (L0 + LN) / 2, B = (L0 - LN) / 2: at K = 5, 27 FP64 instructions per
-// line and field instead of the 35 of K per-node sums with two lift terms.
-template <int K>
-struct LineEOAxis {
-    static constexpr int H = K / 2;
-    double E[H][H], O[H][H];
-    double Dc[H];          // D[i][H], K odd
-    double Al[H], Bl[H];   // lift combinations
-    double Dm[H];          // D[H][j], K odd
-    double Lm;             // L0[H], K odd
-};
-template <int K>
-struct LineEO {
-    LineEOAxis<K> ax[3];
-};
-
-// One line of one field.  The line owners of a warp cover more than one axis
-// (3 K^2 tasks packed densely), so the axis is a runtime value and its
-// coefficients X come from shared memory: every lane runs the same FP64
-// instructions.
-template <int K, int SIG>
-__device__ __forceinline__ void eo_apply(const LineEOAxis<K>& X, const double v[K], double f0, double fN,
-                                         double out[K])
-{
-    constexpr int H = K / 2;
-    double e[H], o[H];
-#pragma unroll
-    for (int j = 0; j < H; j++) {
-        e[j] = v[j] + v[K - 1 - j];
-        o[j] = v[j] - v[K - 1 - j];
-    }
-    const double s = f0 + fN, d = f0 - fN;
-#pragma unroll
-    for (int i = 0; i < H; i++) {
-        double P = X.E[i][0] * e[0], Q = X.O[i][0] * o[0];
-#pragma unroll
-        for (int j = 1; j < H; j++) {
-            P += X.E[i][j] * e[j];
-            Q += X.O[i][j] * o[j];
-        }
-        if (K & 1) P += X.Dc[i] * v[H];
-        if (SIG > 0) {
-            P += X.Bl[i] * d;
-            Q += X.Al[i] * s;
-        } else {
-            P += X.Al[i] * s;
-            Q += X.Bl[i] * d;
-        }
-        out[i] = P + Q;
-        out[K - 1 - i] = Q - P;
-    }
-    if (K & 1) {
-        double c = X.Lm * (SIG > 0 ? s : d);
-#pragma unroll
-        for (int j = 0; j < H; j++) c += X.Dm[j] * o[j];
-        out[H] = c;
-    }
-}
-
 // Line owner with its own face terms (FP32, K >= 5): the two ends of line t
 // along axis A are the face nodes (A, 0, t) and (A, 1, t), so the owner
 // evaluates both numerical fluxes itself (neighbour values ro/uo/qo[side],
@@ -613,80 +546,11 @@ ldg_gradient_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict
     }
 }
 
-// FP64 LDG gradient with even-odd line owners (K = 4, 5: eo_grad_lines): two
-// elements per CTA so that the 3 K^2 line tasks of each pack densely into
-// warps; each owner loads the neighbour values at its line's two ends, forms
-// the central face sums, applies the even-odd operator and stores its line's
-// K results of G_a itself (every value of G has exactly one owner), so the
-// kernel has one barrier, after the element's values reach shared memory,
-// and the threads without a line leave at it.  The stores along y- and
-// z-lines are strided; the kernel is bound by the FP64 pipe, not by memory.
-// Orders whose FP64 stage kernel uses even-odd line owners, by measurement on
-// ~32.8 M nodes of config 2's physics (ms per launch, owners against per-node
-// sums): K = 2: 8.99 / 11.71 (the per-node form leaves 24 of a warp slice's
-// 32 lanes idle); K = 3: 4.49 / 4.57; K = 4: 3.891 / 3.845 (slower); K = 5:
-// 3.85 / 4.12; K = 6 no faster (448-thread CTAs at 92 registers).
-template <int K>
-__host__ __device__ constexpr bool eo_lines()
-{
-    return K <= 3 || K == 5;
-}
-
-// The same choice for the gradient kernel (ms per launch): K = 2: 1.54 /
-// 2.94; K = 3: 1.100 / 1.153; K = 4: 1.106 / 1.122; K = 5: 1.11 / 1.31;
-// K = 6, 7, 8 slower (1.59 / 1.40, 1.73 / 1.60, 2.48 / 1.68).
-template <int K>
-__host__ __device__ constexpr bool eo_grad_lines()
-{
-    return K <= 5;
-}
-
-template <int K>
-__device__ __forceinline__ void grad_eo_line(const LineEOAxis<K>& X, const GradSmem<double, K>& S, int a, int t,
-                                             const double ro[2], double* __restrict__ q_elem)
-{
-    const int st = axis_stride<K>(a);
-    const int b0 = a == 0 ? t : (a == 1 ? (t % K) * K * K + t / K : t * K);
-    double v[K], out[K];
-#pragma unroll
-    for (int j = 0; j < K; j++) v[j] = S.r[b0 + j * st];
-    eo_apply<K, -1>(X, v, ro[0] + v[0], ro[1] + v[K - 1], out);  // flux factors are in the lift columns
-#pragma unroll
-    for (int i = 0; i < K; i++) q_elem[b0 + i * st] = out[i];
-}
-
-template <int K>
-__global__ void __launch_bounds__(npt_of(K) * 2)
-ldg_gradient_eo_kernel(StageIO<double> io, MeshDev<double> m, const OpConst<double, K>* __restrict__ Cp,
-                       const LineEO<K> L)
-{
-    constexpr int K2 = K * K, K3 = K2 * K, NPT = npt_of(K), EPB = 2, NL = 3 * K2;
-    static_assert(NL <= NPT, "line tasks must fit the element's threads");
-    __shared__ GradSmem<double, K> sm_all[EPB];
-    __shared__ LineEOAxis<K> eo[3];
-    const OpConst<double, K>& C = *Cp;
-    const int n = threadIdx.x;
-    const int e = blockIdx.x * EPB + threadIdx.y;
-    const bool act = n < K3 && e < m.n_elem;
-    if (threadIdx.y == 0 && n < 3) eo[n] = n == 0 ? L.ax[0] : (n == 1 ? L.ax[1] : L.ax[2]);
-    // this thread's line task: element le of the CTA, axis la, line t
-    const int tid = threadIdx.y * NPT + n;
-    const int le = tid / NL, la = (tid % NL) / K2, t = tid % K2;
-    const int el = blockIdx.x * EPB + le;
-    const bool owner = tid < EPB * NL && el < m.n_elem;
-    double rho = 0.0, ro[2] = {0.0, 0.0}, unused_u[2], unused_q[2];
-    if (act) rho = __ldg(io.src + (size_t)e * io.np + n);
-    if (owner) line_end_values<false, false, false, double, K>(io, m, C, el, la, t, ro, unused_u, unused_q);
-    sm_all[threadIdx.y].r[n] = rho;
-    __syncthreads();
-    if (owner) grad_eo_line<K>(eo[la], sm_all[le], la, t, ro, io.q_out + (size_t)la * io.fs + (size_t)el * io.np);
-}
-
 // Shared memory of a stage kernel, per element: for each axis a, the pair
 // (f_mom, f_mass along a + G_a) of every node (one 8- or 16-byte load feeds
 // two FMAs of a line sum), the pair (momentum, density) of every face term
 // [axis][side][face node], and each node's own mass flux and gradient, which
-// the face phase reads (and the line owners then reuse for their results).
+// the face phase reads (and the FP32 line owners then reuse for their results).
 template <typename T, int K>
 struct PlainSmem {
     typename Pair<T>::type f[3][npt_of(K)];
@@ -699,58 +563,14 @@ struct PlainSmem {
 // One RK stage of the plain (FP64) form: R = L(stage input), then the stage
 // combination dst = R' + s (cb - ca sigma) + cc old.
 //
-// The FP64 pipe is the bound, so the face fluxes are assigned densely: with
-// per-node line sums, thread n of an element evaluates face nodes n, n + NPT,
-// ... of its 6 K^2, reading the element's own values from shared memory; with
-// even-odd line owners, each owner evaluates the two face nodes that end its
-// line (the line tasks are packed densely too).  (A thread per node evaluating
-// its own faces would issue every axis's face arithmetic in nearly every warp,
-// since almost every warp holds some node on each face pair.)  The neighbour
-// values of those face nodes are loaded with the thread's own node.
+// Per-node FP64 sums, for operators without a fixed-point form (see
+// fix_kernels.cuh).  The face fluxes are assigned densely: thread n of an
+// element evaluates face nodes n, n + NPT, ... of its 6 K^2, reading the
+// element's own values from shared memory (a thread per node evaluating its
+// own faces would issue every axis's face arithmetic in nearly every warp).
+// The neighbour values of those face nodes are loaded with the thread's own
+// node.
 // ---------------------------------------------------------------------------
-// Elements per CTA of the FP64 stage kernel: two with even-odd line owners
-// (EO), so that the 3 K^2 line tasks of each pack densely into warps.
-template <int K, bool EO>
-__host__ __device__ constexpr int plain_epb()
-{
-    return EO ? 2 : epb_of(K);
-}
-
-// Resident CTAs per SM asked of the compiler for the FP64 stage kernel (0:
-// no request): at K = 5, 64 registers keep 32 warps per SM.
-template <typename T, int K, bool EO>
-__host__ __device__ constexpr int plain_min_blocks()
-{
-    return (sizeof(T) == 8 && K == 5) ? 8 / plain_epb<K, EO>() : 0;
-}
-
-// One line of an FP64 stage kernel with even-odd line owners: the mass
-// equation's line (flux f_mass + G, face terms gr) into S.m and the momentum
-// equation's (f_mom, gm) into S.q, along runtime axis a.
-// The line's face terms g0 (first node) and gN (last node) come from its
-// owner (x momentum, y density).
-template <int K>
-__device__ __forceinline__ void stage_eo_line(const LineEOAxis<K>& X, PlainSmem<double, K>& S, int a, int t,
-                                              int do_adv, const double2 g0, const double2 gN)
-{
-    const int st = axis_stride<K>(a);
-    const int b0 = a == 0 ? t : (a == 1 ? (t % K) * K * K + t / K : t * K);
-    // one field at a time (fewer live registers than both at once)
-    double v[K], out[K];
-#pragma unroll
-    for (int j = 0; j < K; j++) v[j] = S.f[a][b0 + j * st].y;
-    eo_apply<K, 1>(X, v, g0.y, gN.y, out);
-#pragma unroll
-    for (int i = 0; i < K; i++) S.m[a][b0 + i * st] = out[i];
-    if (do_adv) {
-#pragma unroll
-        for (int j = 0; j < K; j++) v[j] = S.f[a][b0 + j * st].x;
-        eo_apply<K, 1>(X, v, g0.x, gN.x, out);
-#pragma unroll
-        for (int i = 0; i < K; i++) S.q[a][b0 + i * st] = out[i];
-    }
-}
-
 // Face term (x momentum, y density) of face node nf of an element on axis a,
 // side ``side``: the numerical flux (impedance upwind for advection, central
 // for LDG) times its lift scale, from the element's own values in shared
@@ -788,23 +608,13 @@ __device__ __forceinline__ typename Pair<T>::type face_term(const OpConst<T, K>&
 // of evaluating every interior face node's neighbour flux a second time
 // (its own element evaluates it for its line sums).
 //
-// Line sums (EO): false, every node sums its three lines itself (operator
-// rows in registers); true (D centro-antisymmetric, see LineEO), line owners
-// apply the even-odd operator after the face phase, one more barrier, and
-// each node adds its three axis results.
-//
-// PACK: the stage's output is also written in host order to io.pack (the
-// last stage of a step whose result is downloaded: the pack rides on the
-// FP64-bound stage instead of a kernel of its own).
-template <typename T, int K, bool DIFF, int FLUX, bool EO, bool PACK = false>
-__global__ void __launch_bounds__(npt_of(K) * plain_epb<K, EO>(), (plain_min_blocks<T, K, EO>()))
-stage_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__ Cp, const LineEO<K> L, int do_adv,
-             int do_sponge)
+template <typename T, int K, bool DIFF, int FLUX>
+__global__ void __launch_bounds__(npt_of(K) * epb_of(K))
+stage_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__ Cp, int do_adv, int do_sponge)
 {
     constexpr int K2 = K * K, K3 = K * K * K, NPT = npt_of(K), NF = 6 * K2, R = (NF + NPT - 1) / NPT;
-    constexpr int EPB = plain_epb<K, EO>();
+    constexpr int EPB = epb_of(K);
     __shared__ PlainSmem<T, K> sm_all[EPB];
-    __shared__ LineEOAxis<K> eo[EO ? 3 : 1];
     PlainSmem<T, K>& S = sm_all[threadIdx.y];
     const OpConst<T, K>& C = *Cp;
     const int n = threadIdx.x;
@@ -814,11 +624,7 @@ stage_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__ Cp, 
     const int c[3] = {n / K2, (n / K) % K, n % K};
     const size_t off = (size_t)e * io.np + n;
     OpRows<T, K> R_;
-    if constexpr (EO) {
-        if (threadIdx.y == 0 && n < 3) eo[n] = n == 0 ? L.ax[0] : (n == 1 ? L.ax[1] : L.ax[2]);
-    } else {
-        R_.load(C, c, act);
-    }
+    R_.load(C, c, act);
 
     T rho = T(0), u[3] = {T(0), T(0), T(0)}, q[3] = {T(0), T(0), T(0)};
     T fl[4] = {T(0), T(0), T(0), T(0)};
@@ -837,51 +643,27 @@ stage_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__ Cp, 
     }
     // Neighbour (or exterior) values of this thread's face nodes: drho and
     // the normal velocity, or in flux mode 2 their momentum and mass fluxes.
-    // Per-node line sums: the element's 6 K^2 face nodes dealt out densely
-    // (slots n, n + NPT, ...).  EO: the two ends of this thread's line task
-    // (element le of the CTA, axis la, line lt), whose face terms its owner
-    // evaluates itself, so the face phase needs no barrier of its own.
-    constexpr int NL = 3 * K2, RF = EO ? 2 : R;
-    const int tid = threadIdx.y * NPT + n;
-    const int le = tid / NL, la = (tid % NL) / K2, lt = tid % K2;
-    const bool owner = EO && tid < EPB * NL && blockIdx.x * EPB + le < m.n_elem;
-    T ro[RF], uo[RF], qo[RF];
+    // The element's 6 K^2 face nodes are dealt out densely (slots n, n + NPT, ...).
+    T ro[R], uo[R], qo[R];
 #pragma unroll
-    for (int r = 0; r < RF; r++) {
+    for (int r = 0; r < R; r++) {
         ro[r] = uo[r] = qo[r] = T(0);
-        int fa, fside, ffi, fnn, fe;
-        if constexpr (EO) {
-            if (!owner) continue;
-            const int st = axis_stride<K>(la);
-            const int b0 = la == 0 ? lt : (la == 1 ? (lt % K) * K2 + lt / K : lt * K);
-            fa = la;
-            fside = r;
-            ffi = lt;
-            fnn = b0 + (r ? 0 : (K - 1) * st);
-            fe = blockIdx.x * EPB + le;
-        } else {
-            const int t = n + r * NPT;
-            if (!live || t >= NF) continue;
-            const FaceNode<K> F(t);
-            fa = F.a;
-            fside = F.side;
-            ffi = F.fi;
-            fnn = F.nn;
-            fe = e;
-        }
-        const int code = __ldg(m.nbr + (size_t)fe * 6 + 2 * fa + fside);
+        const int t = n + r * NPT;
+        if (!live || t >= NF) continue;
+        const FaceNode<K> F(t);
+        const int code = __ldg(m.nbr + (size_t)e * 6 + 2 * F.a + F.side);
         if (code >= 0) {
-            const size_t o2 = (size_t)code * io.np + fnn;
+            const size_t o2 = (size_t)code * io.np + F.nn;
             if (FLUX == 2) {
                 ro[r] = __ldg(io.flux_in + o2);
-                uo[r] = __ldg(io.flux_in + (size_t)(1 + fa) * io.fs + o2);
+                uo[r] = __ldg(io.flux_in + (size_t)(1 + F.a) * io.fs + o2);
             } else {
                 ro[r] = load_in<false>(io, 0, o2);
-                uo[r] = load_in<false>(io, 1 + fa, o2);
+                uo[r] = load_in<false>(io, 1 + F.a, o2);
             }
-            if (DIFF) qo[r] = __ldg(io.q + (size_t)fa * io.fs + o2);
+            if (DIFF) qo[r] = __ldg(io.q + (size_t)F.a * io.fs + o2);
         } else {
-            exterior<T, K>(m, C, -1 - code, fside, ffi, ro[r], uo[r]);
+            exterior<T, K>(m, C, -1 - code, F.side, F.fi, ro[r], uo[r]);
             if (FLUX == 2) {
                 const T fm = momentum_flux(ro[r], C.k1, C.k2);
                 uo[r] = mass_flux(uo[r], ro[r], C.r0, C.linear_mass);
@@ -909,60 +691,37 @@ stage_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__ Cp, 
     }
     __syncthreads();
 
-    // Face terms (dense form): the numerical flux times its lift scale.
-    if constexpr (!EO) {
+    // Face terms: the numerical flux times its lift scale.
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-            const int t = n + r * NPT;
-            if (!live || t >= NF) continue;
-            const FaceNode<K> F(t);
-            S.g[F.a][F.side][F.fi] = face_term<T, K, DIFF, FLUX>(C, S, F.a, F.side, F.nf, ro[r], uo[r], qo[r], do_adv);
-        }
-        __syncthreads();
+    for (int r = 0; r < R; r++) {
+        const int t = n + r * NPT;
+        if (!live || t >= NF) continue;
+        const FaceNode<K> F(t);
+        S.g[F.a][F.side][F.fi] = face_term<T, K, DIFF, FLUX>(C, S, F.a, F.side, F.nf, ro[r], uo[r], qo[r], do_adv);
     }
-
-    T r_rho = T(0), r_u[3] = {T(0), T(0), T(0)};
-    if constexpr (EO) {
-        static_assert(NL <= NPT, "line tasks must fit the element's threads");
-        if (owner) {
-            PlainSmem<T, K>& SL = sm_all[le];
-            const int st = axis_stride<K>(la);
-            const int b0 = la == 0 ? lt : (la == 1 ? (lt % K) * K2 + lt / K : lt * K);
-            const typename Pair<T>::type g0 = face_term<T, K, DIFF, FLUX>(C, SL, la, 0, b0, ro[0], uo[0], qo[0], do_adv);
-            const typename Pair<T>::type gN =
-                face_term<T, K, DIFF, FLUX>(C, SL, la, 1, b0 + (K - 1) * st, ro[1], uo[1], qo[1], do_adv);
-            stage_eo_line<K>(eo[la], SL, la, lt, do_adv, g0, gN);
-        }
-        __syncthreads();
-        if (!act) return;
-        r_rho = S.m[0][n] + S.m[1][n];
-        r_rho += S.m[2][n];
-#pragma unroll
-        for (int a = 0; a < 3; a++) r_u[a] = do_adv ? S.q[a][n] : T(0);
-    }
+    __syncthreads();
     if (!act) return;
 
-    if constexpr (!EO) {
-        // The density equation is one FMA chain through the three axes (no
-        // per-axis partial sums to add): the kernel is bound by FP64 issue,
-        // so every FP64 instruction saved per node counts.
+    // The density equation is one FMA chain through the three axes (no
+    // per-axis partial sums to add): the kernel is bound by FP64 issue, so
+    // every FP64 instruction saved per node counts.
+    T r_rho = T(0), r_u[3] = {T(0), T(0), T(0)};
 #pragma unroll
-        for (int a = 0; a < 3; a++) {
-            const int st = axis_stride<K>(a), base = n - c[a] * st;
-            const int fi = c[(a + 1) % 3] * K + c[(a + 2) % 3];
-            const typename Pair<T>::type g0 = S.g[a][0][fi], gN = S.g[a][1][fi];
-            T sm = R_.l0[a] * g0.x;
-            sm += R_.ln[a] * gN.x;
-            r_rho += R_.l0[a] * g0.y;
-            r_rho += R_.ln[a] * gN.y;
+    for (int a = 0; a < 3; a++) {
+        const int st = axis_stride<K>(a), base = n - c[a] * st;
+        const int fi = c[(a + 1) % 3] * K + c[(a + 2) % 3];
+        const typename Pair<T>::type g0 = S.g[a][0][fi], gN = S.g[a][1][fi];
+        T sm = R_.l0[a] * g0.x;
+        sm += R_.ln[a] * gN.x;
+        r_rho += R_.l0[a] * g0.y;
+        r_rho += R_.ln[a] * gN.y;
 #pragma unroll
-            for (int j = 0; j < K; j++) {
-                const typename Pair<T>::type v = S.f[a][base + j * st];
-                sm += R_.d[a][j] * v.x;
-                r_rho += R_.d[a][j] * v.y;
-            }
-            r_u[a] = do_adv ? sm : T(0);
+        for (int j = 0; j < K; j++) {
+            const typename Pair<T>::type v = S.f[a][base + j * st];
+            sm += R_.d[a][j] * v.x;
+            r_rho += R_.d[a][j] * v.y;
         }
+        r_u[a] = do_adv ? sm : T(0);
     }
     // cb - ca sigma of this element: tabulated per stage by the host, so that
     // no thread spends FP64 instructions on it; computed here when absent.
@@ -990,11 +749,6 @@ stage_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__ Cp, 
 #pragma unroll
         for (int a = 0; a < 3; a++)
             io.flux_out[(size_t)(1 + a) * io.fs + off] = mass_flux(vo[1 + a], vo[0], C.r0, C.linear_mass);
-    }
-    if constexpr (PACK) {
-        const size_t gi = grid_index(io.pack_map, e, n);
-#pragma unroll
-        for (int f = 0; f < 4; f++) io.pack[(size_t)f * io.pack_gsize + gi] = (double)vo[f];
     }
 }
 
@@ -1264,41 +1018,6 @@ inline OpConst<T, K> make_grad_const(const double* deriv, const double* lift0, c
     C.inv_c2 = (T)(1.0 / (c0 * c0));
     C.inv_z = (T)(1.0 / (rho0 * c0));
     return C;
-}
-
-// Even-odd split of the per-axis rows of C (see LineEO); false when D is not
-// centro-antisymmetric or the lift columns are not mirrored with sign SIG, to
-// 1e-12 of their largest entry, and the line owners must not be used.
-template <int K, int SIG>
-inline bool make_line_eo(const OpConst<double, K>& C, LineEO<K>& L)
-{
-    constexpr int H = K / 2;
-    if (H < 1) return false;
-    for (int a = 0; a < 3; a++) {
-        const auto& R = C.rows[a];
-        double dmax = 0.0, lmax = 0.0;
-        for (int i = 0; i < K; i++) {
-            for (int j = 0; j < K; j++) dmax = std::fmax(dmax, std::fabs(R[i][j]));
-            lmax = std::fmax(lmax, std::fmax(std::fabs(R[i][K]), std::fabs(R[i][K + 1])));
-        }
-        for (int i = 0; i < K; i++) {
-            for (int j = 0; j < K; j++)
-                if (std::fabs(R[i][j] + R[K - 1 - i][K - 1 - j]) > 1e-12 * dmax) return false;
-            if (std::fabs(R[K - 1 - i][K] - SIG * R[i][K + 1]) > 1e-12 * lmax) return false;
-        }
-        for (int i = 0; i < H; i++) {
-            for (int j = 0; j < H; j++) {
-                L.ax[a].E[i][j] = 0.5 * (R[i][j] + R[i][K - 1 - j]);
-                L.ax[a].O[i][j] = 0.5 * (R[i][j] - R[i][K - 1 - j]);
-            }
-            L.ax[a].Dc[i] = (K & 1) ? R[i][H] : 0.0;
-            L.ax[a].Al[i] = 0.5 * (R[i][K] + R[i][K + 1]);
-            L.ax[a].Bl[i] = 0.5 * (R[i][K] - R[i][K + 1]);
-            L.ax[a].Dm[i] = (K & 1) ? R[H][i] : 0.0;
-        }
-        L.ax[a].Lm = (K & 1) ? R[H][K] : 0.0;
-    }
-    return true;
 }
 
 // State <-> host-order arrays rho [X][Y][Z], vel [3][X][Y][Z], walked in host

@@ -21,10 +21,10 @@
 // so a cudaDeviceReset of a device invalidates it (this entry point is not
 // for processes that reset devices while it is loaded).  Every call shares the
 // array and it keeps the last call's contents: the gradient part is fully
-// rewritten by each call before it is read, the boundary-flag part is cleared
-// by each call, the operator part is rewritten by each call, and calls whose
-// work overlaps on the same GPU (for example calls issued to two streams with
-// no ordering between them) race on it.
+// rewritten by each call before it is read, the boundary-flag and operator
+// parts are rewritten by each call that reads them, and calls whose work
+// overlaps on the same GPU (for example calls issued to two streams with no
+// ordering between them) race on it.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -34,6 +34,7 @@
 
 #include "dg3d.h"
 #include "dg_kernels.cuh"
+#include "fix_kernels.cuh"
 #include "solver_internal.h"
 
 namespace {
@@ -46,7 +47,8 @@ constexpr size_t kConstSlot = 4096;  // one per-launch operator (OpConst<double,
 
 // LDG gradient (3 x kMaxSlots doubles), the boundary-source flags (6 x
 // kMaxElems ints, zero: every boundary face reads a zero exterior state) and
-// two operator slots (stage, gradient).
+// two operator slots (stage, gradient); the last two serve the kernels without
+// a fixed-point operator.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kQBytes + kFlagBytes + 2 * kConstSlot];
 
 constexpr int kMaxDevices = 64;
@@ -133,26 +135,43 @@ __global__ void store_operators_kernel(dg::OpConst<double, K>* __restrict__ dst,
 
 template <int K>
 cudaError_t launch(const dg_params& p, const double* D, const double* L0, const double* LN,
-                   const dg::StageIO<double>& io, const dg::MeshDev<double>& md, unsigned char* consts,
-                   cudaStream_t st)
+                   const dg::StageIO<double>& io, const dg::MeshDev<double>& md, int* flags,
+                   unsigned char* consts, cudaStream_t st)
 {
     static_assert(sizeof(dg::OpConst<double, K>) <= kConstSlot, "operator slot too small");
     const dg::OpConst<double, K> C = dg::make_stage_const<double, K>(1.0, D, L0, LN, p.elem_width, p.rho0, p.c0,
                                                                      p.b_over_a, p.diff_const);
     const dg::OpConst<double, K> G =
         dg::make_grad_const<double, K>(D, L0, LN, p.elem_width, p.rho0, p.c0, p.diff_const);
-    store_operators_kernel<K><<<1, 128, 0, st>>>((dg::OpConst<double, K>*)consts, C, G);
+    dg::FixOps<K, 2> FC;
+    dg::FixOps<K, 1> FG;
+    const bool fix = dg::make_stage_fix<K>(C, FC), fix_grad = dg::make_grad_fix<K>(G, FG);
+    // the fixed-point kernels take their operators as parameters and no
+    // boundary tables as zero outside; the others read both from the scratch
+    if (!fix || (p.eval_diff && !fix_grad)) {
+        const cudaError_t e = cudaMemsetAsync(flags, 0, (size_t)6 * md.n_elem * sizeof(int), st);
+        if (e != cudaSuccess) return e;
+        store_operators_kernel<K><<<1, 128, 0, st>>>((dg::OpConst<double, K>*)consts, C, G);
+    }
+    dg::MeshDev<double> mf = md;
+    mf.bnd_src = nullptr;
     const dg::OpConst<double, K>* Cd = (const dg::OpConst<double, K>*)consts;
     const dg::OpConst<double, K>* Gd = (const dg::OpConst<double, K>*)(consts + kConstSlot);
-    dim3 block(dg::npt_of(K), dg::epb_of(K));
-    dim3 grid((md.n_elem + dg::epb_of(K) - 1) / dg::epb_of(K));
+    const dim3 block(dg::npt_of(K), dg::epb_of(K));
+    const int grid = (md.n_elem + dg::epb_of(K) - 1) / dg::epb_of(K);
+    const int fix_grid = (md.n_elem + dg::fix_epb(K) - 1) / dg::fix_epb(K);
     if (p.eval_diff) {
-        dg::ldg_gradient_kernel<double, K, false><<<grid, block, 0, st>>>(io, md, Gd, G);
-        dg::stage_kernel<double, K, true, 0, false><<<grid, block, 0, st>>>(io, md, Cd, dg::LineEO<K>{}, p.eval_advect,
-                                                                          p.eval_sponge);
+        if (fix_grad) dg::ldg_gradient_fix_kernel<K><<<fix_grid, dg::fix_threads(K), 0, st>>>(io, mf, G, FG);
+        else dg::ldg_gradient_kernel<double, K, false><<<grid, block, 0, st>>>(io, md, Gd, G);
+        if (fix)
+            dg::stage_fix_kernel<K, true, 0, false>
+                <<<fix_grid, dg::fix_threads(K), 0, st>>>(io, mf, C, FC, p.eval_advect, p.eval_sponge);
+        else dg::stage_kernel<double, K, true, 0><<<grid, block, 0, st>>>(io, md, Cd, p.eval_advect, p.eval_sponge);
     } else {
-        dg::stage_kernel<double, K, false, 0, false><<<grid, block, 0, st>>>(io, md, Cd, dg::LineEO<K>{}, p.eval_advect,
-                                                                          p.eval_sponge);
+        if (fix)
+            dg::stage_fix_kernel<K, false, 0, false>
+                <<<fix_grid, dg::fix_threads(K), 0, st>>>(io, mf, C, FC, p.eval_advect, p.eval_sponge);
+        else dg::stage_kernel<double, K, false, 0><<<grid, block, 0, st>>>(io, md, Cd, p.eval_advect, p.eval_sponge);
     }
     return cudaSuccess;
 }
@@ -188,8 +207,7 @@ extern "C" int dg_eval_rhs_noalloc(const dg_params* p, const double* mass, const
     double* q = (double*)scratch;
     int* flags = (int*)((unsigned char*)scratch + kQBytes);
     unsigned char* consts = (unsigned char*)scratch + kQBytes + kFlagBytes;
-    cudaError_t e = cudaMemsetAsync(flags, 0, (size_t)6 * n_elem * sizeof(int), st);
-    if (e != cudaSuccess) return dg::fail(DG_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
+    cudaError_t e = cudaSuccess;
 
     dg::StageIO<double> io;
     std::memset(&io, 0, sizeof io);
@@ -211,13 +229,13 @@ extern "C" int dg_eval_rhs_noalloc(const dg_params* p, const double* mass, const
     md.ic_live = 0;
     md.src_p = 0.0;
     switch (K) {
-    case 2: e = launch<2>(*p, D, L0, LN, io, md, consts, st); break;
-    case 3: e = launch<3>(*p, D, L0, LN, io, md, consts, st); break;
-    case 4: e = launch<4>(*p, D, L0, LN, io, md, consts, st); break;
-    case 5: e = launch<5>(*p, D, L0, LN, io, md, consts, st); break;
-    case 6: e = launch<6>(*p, D, L0, LN, io, md, consts, st); break;
-    case 7: e = launch<7>(*p, D, L0, LN, io, md, consts, st); break;
-    case 8: e = launch<8>(*p, D, L0, LN, io, md, consts, st); break;
+    case 2: e = launch<2>(*p, D, L0, LN, io, md, flags, consts, st); break;
+    case 3: e = launch<3>(*p, D, L0, LN, io, md, flags, consts, st); break;
+    case 4: e = launch<4>(*p, D, L0, LN, io, md, flags, consts, st); break;
+    case 5: e = launch<5>(*p, D, L0, LN, io, md, flags, consts, st); break;
+    case 6: e = launch<6>(*p, D, L0, LN, io, md, flags, consts, st); break;
+    case 7: e = launch<7>(*p, D, L0, LN, io, md, flags, consts, st); break;
+    case 8: e = launch<8>(*p, D, L0, LN, io, md, flags, consts, st); break;
     }
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return dg::fail(DG_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));

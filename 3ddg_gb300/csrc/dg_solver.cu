@@ -13,6 +13,7 @@
 #include "basis.h"
 #include "dg3d.h"
 #include "dg_kernels.cuh"
+#include "fix_kernels.cuh"
 #include "mesh.h"
 #include "solver_internal.h"
 
@@ -89,9 +90,22 @@ double stage_flops(const Solver& s, bool has_old)
 // three RK stages, the LDG gradient and a bare right-hand side), rebuilt
 // only when dt changes.
 template <typename T, int K>
-size_t const_slot()
+constexpr size_t const_slot()
 {
     return (sizeof(OpConst<T, K>) + 255) / 256 * 256;
+}
+
+// Fixed-point forms of the FP64 operators, kept on the host: they travel as
+// kernel parameters.
+template <int K>
+struct FixSet {
+    FixOps<K, 2> stage[5];  // 3 RK stages, -, bare right-hand side
+    FixOps<K, 1> grad;
+};
+template <int K>
+const FixSet<K>& fix_set(const Solver& s)
+{
+    return *(const FixSet<K>*)s.h_fix.data();
 }
 
 template <typename T, int K>
@@ -107,6 +121,11 @@ int upload_consts_k(Solver& s, double dt)
                    : make_stage_const<T, K>(cas[i], s.op.deriv.data(), s.op.lift0.data(), s.op.liftN.data(),
                                             s.p.elem_width, s.p.rho0, s.p.c0, s.p.b_over_a, s.p.diff_const);
         std::memcpy(h.data() + i * slot, &C, sizeof C);
+        if constexpr (sizeof(T) == 8) {
+            s.h_fix.resize(sizeof(FixSet<K>));
+            FixSet<K>& F = *(FixSet<K>*)s.h_fix.data();
+            s.fix_ok[i] = i == 3 ? make_grad_fix<K>(C, F.grad) : make_stage_fix<K>(C, F.stage[i]);
+        }
     }
     if (!s.d_const) {
         cudaError_t e = cudaMalloc(&s.d_const, 5 * slot);
@@ -140,11 +159,10 @@ void launch_grad(Solver& s, const StageIO<T>& io, const MeshDev<T>& md)
     cudaEvent_t ev = nullptr;
     s.prof_begin(1, &ev);
     bool done = false;
-    if constexpr (!INCR && sizeof(T) == 8 && eo_grad_lines<K>()) {
-        LineEO<K> L;
-        if (make_line_eo<K, -1>(host_const<T, K>(s, 3), L)) {
-            ldg_gradient_eo_kernel<K><<<(md.n_elem + 1) / 2, dim3(npt_of(K), 2), 0, s.stream>>>(
-                io, md, const_ptr<T, K>(s, 3), L);
+    if constexpr (!INCR && sizeof(T) == 8) {
+        if (s.fix_ok[3]) {
+            ldg_gradient_fix_kernel<K><<<(md.n_elem + fix_epb(K) - 1) / fix_epb(K), fix_threads(K), 0, s.stream>>>(
+                io, md, host_const<T, K>(s, 3), fix_set<K>(s).grad);
             done = true;
         }
     }
@@ -156,54 +174,44 @@ void launch_grad(Solver& s, const StageIO<T>& io, const MeshDev<T>& md)
 }
 
 // FP64 stage kernel in the flux mode that io asks for (flux_out: write the
-// output's volume fluxes; flux_in: read the input's), with even-odd line
-// owners where the order has them and the operator allows them.
-template <typename T, int K, bool DIFF, bool EO, int FLUX, bool PACK = false>
-void launch_plain_eo(const Solver& s, const StageIO<T>& io, const MeshDev<T>& md, const OpConst<T, K>* Cp,
-                     const LineEO<K>& L)
+// output's volume fluxes; flux_in: read the input's): the fixed-point kernel
+// where the operator has that form, else the per-node FP64 sums.
+template <int K, bool DIFF, int FLUX, bool PACK = false>
+void launch_plain_mode(const Solver& s, int slot, const StageIO<double>& io, const MeshDev<double>& md)
 {
-    const dim3 block(npt_of(K), plain_epb<K, EO>());
-    const dim3 grid((md.n_elem + plain_epb<K, EO>() - 1) / plain_epb<K, EO>());
-    stage_kernel<T, K, DIFF, FLUX, EO, PACK><<<grid, block, 0, s.stream>>>(io, md, Cp, L, s.p.eval_advect,
-                                                                          s.p.eval_sponge);
+    if (s.fix_ok[slot])
+        stage_fix_kernel<K, DIFF, FLUX, PACK>
+            <<<(md.n_elem + fix_epb(K) - 1) / fix_epb(K), fix_threads(K), 0, s.stream>>>(
+                io, md, host_const<double, K>(s, slot), fix_set<K>(s).stage[slot], s.p.eval_advect, s.p.eval_sponge);
+    else
+        stage_kernel<double, K, DIFF, FLUX>
+            <<<(md.n_elem + epb_of(K) - 1) / epb_of(K), dim3(npt_of(K), epb_of(K)), 0, s.stream>>>(
+                io, md, const_ptr<double, K>(s, slot), s.p.eval_advect, s.p.eval_sponge);
 }
 
 // The host-order pack rides only on the flux-reading mode (the steady state
-// of stepping with advection); io.pack is set only when that mode runs.
-template <typename T, int K, bool DIFF, bool EO>
-void launch_plain_mode(const Solver& s, const StageIO<T>& io, const MeshDev<T>& md, const OpConst<T, K>* Cp,
-                       const LineEO<K>& L)
+// of stepping with advection) of the fixed-point kernel; io.pack is set only
+// when that runs.
+template <int K, bool DIFF>
+void launch_plain(const Solver& s, int slot, const StageIO<double>& io, const MeshDev<double>& md)
 {
     if (io.flux_out && io.flux_in) {
-        if (io.pack) launch_plain_eo<T, K, DIFF, EO, 2, true>(s, io, md, Cp, L);
-        else launch_plain_eo<T, K, DIFF, EO, 2>(s, io, md, Cp, L);
+        if (io.pack) launch_plain_mode<K, DIFF, 2, true>(s, slot, io, md);
+        else launch_plain_mode<K, DIFF, 2>(s, slot, io, md);
     } else if (io.flux_out) {
-        launch_plain_eo<T, K, DIFF, EO, 1>(s, io, md, Cp, L);
+        launch_plain_mode<K, DIFF, 1>(s, slot, io, md);
     } else {
-        launch_plain_eo<T, K, DIFF, EO, 0>(s, io, md, Cp, L);
+        launch_plain_mode<K, DIFF, 0>(s, slot, io, md);
     }
-}
-
-template <typename T, int K, bool DIFF>
-void launch_plain(const Solver& s, int slot, const StageIO<T>& io, const MeshDev<T>& md, const OpConst<T, K>* Cp)
-{
-    LineEO<K> L{};
-    if constexpr (sizeof(T) == 8 && eo_lines<K>()) {
-        if (make_line_eo<K, 1>(host_const<T, K>(s, slot), L)) {
-            launch_plain_mode<T, K, DIFF, true>(s, io, md, Cp, L);
-            return;
-        }
-    }
-    launch_plain_mode<T, K, DIFF, false>(s, io, md, Cp, L);
 }
 
 template <typename T, int K, bool INCR>
 void launch_stage(Solver& s, const StageIO<T>& io, const MeshDev<T>& md, int slot)
 {
-    const OpConst<T, K>* Cp = const_ptr<T, K>(s, slot);
     cudaEvent_t ev = nullptr;
     s.prof_begin(0, &ev);
     if constexpr (INCR) {
+        const OpConst<T, K>* Cp = const_ptr<T, K>(s, slot);
         const dim3 block(npt_of(K), epb_of(K));
         const dim3 grid((md.n_elem + epb_of(K) - 1) / epb_of(K));
         const OpConst<T, K>& Cv = host_const<T, K>(s, slot);
@@ -214,8 +222,8 @@ void launch_stage(Solver& s, const StageIO<T>& io, const MeshDev<T>& md, int slo
             incr_stage_kernel<T, K, false><<<grid, block, 0, s.stream>>>(io, md, Cp, Cv, s.p.eval_advect,
                                                                         s.p.eval_sponge);
     } else {
-        if (s.p.eval_diff) launch_plain<T, K, true>(s, slot, io, md, Cp);
-        else launch_plain<T, K, false>(s, slot, io, md, Cp);
+        if (s.p.eval_diff) launch_plain<K, true>(s, slot, io, md);
+        else launch_plain<K, false>(s, slot, io, md);
     }
     s.prof_end(0, ev, stage_bytes<T, INCR>(s, io), stage_flops(s, io.old != nullptr || io.inc != nullptr));
     s.launches++;
@@ -371,7 +379,7 @@ int Solver::rk_stage_fp64(int s_idx, double dt, double* rhs_only)
         io.flux_in = flux_valid ? d_flux[flux_cur] : nullptr;
         io.flux_out = d_flux[1 - flux_cur];
     }
-    if (s_idx == 2 && !rhs_only && stage3_pack && io.flux_in && io.flux_out) {
+    if (s_idx == 2 && !rhs_only && stage3_pack && io.flux_in && io.flux_out && fix_ok[s_idx]) {
         io.pack = stage3_pack;
         io.pack_map = grid_map(mesh);
         io.pack_gsize = gsize();

@@ -40,6 +40,8 @@ struct Solver {
     void* d_bnd_ap = nullptr;
     int* d_bnd_src = nullptr;
     void* d_const = nullptr;  // per-launch operators: 3 RK stages, LDG gradient, bare RHS
+    bool fix_ok[5] = {};        // FP64: the operator has a fixed-point form
+    std::vector<char> h_fix;    // FP64: those forms (FixSet of dg_solver.cu)
     std::vector<char> h_const;  // host copy of d_const (for by-value kernel parameters)
     double* d_elem_b = nullptr;  // FP64: cb - ca sigma per element for the 3 RK stages
     // FP64 with advection: volume fluxes (f_mom, f_mass x, y, z) of the next
