@@ -71,6 +71,21 @@ void fill_ops(BatchProblem& P, const LineOperators& op, const dg_params& p)
     P.linear_mass = C.linear_mass;
 }
 
+// A launch whose blocks take few tiles each starts under the one before it in
+// its branch (launch_pdl; with the step bookkeeping in one launch, 8 problems of 4..8 elements per axis 53 -> 43 us per
+// step, one of 6^3 32 -> 20 us); one that streams many has no gap to hide and
+// keeps the read-only loads.  The first launch of a step (``after`` false)
+// reads descriptors that the launch before it wrote, so it waits for it.
+constexpr int kDependentTiles = 2;
+template <int K, int PHASE>
+void launch_batch(const BatchArgs& A, const BatchOps& ops, int grid, bool after, cudaStream_t st)
+{
+    if (after && A.n_tiles <= kDependentTiles * grid)
+        launch_pdl(batch_stage_kernel<K, PHASE, true>, grid, bthreads_of(K), st, A, ops);
+    else
+        batch_stage_kernel<K, PHASE, false><<<grid, bthreads_of(K), 0, st>>>(A, ops);
+}
+
 }  // namespace
 
 // ------------------------------------------------------------ PinnedPool
@@ -173,16 +188,16 @@ int Batch::init(int device_capacity)
     cudaDeviceProp prop;
     DGB_CUDA(cudaGetDeviceProperties(&prop, device));
     num_sms = prop.multiProcessorCount;
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[2][0], batch_stage_kernel<2, 0>, bthreads_of(2), 0));
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[2][1], batch_stage_kernel<2, 1>, bthreads_of(2), 0));
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[3][0], batch_stage_kernel<3, 0>, bthreads_of(3), 0));
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[3][1], batch_stage_kernel<3, 1>, bthreads_of(3), 0));
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[4][0], batch_stage_kernel<4, 0>, bthreads_of(4), 0));
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[4][1], batch_stage_kernel<4, 1>, bthreads_of(4), 0));
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[5][0], batch_stage_kernel<5, 0>, bthreads_of(5), 0));
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[5][1], batch_stage_kernel<5, 1>, bthreads_of(5), 0));
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[6][0], batch_stage_kernel<6, 0>, bthreads_of(6), 0));
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[6][1], batch_stage_kernel<6, 1>, bthreads_of(6), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[2][0], batch_stage_kernel<2, 0, false>, bthreads_of(2), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[2][1], batch_stage_kernel<2, 1, false>, bthreads_of(2), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[3][0], batch_stage_kernel<3, 0, false>, bthreads_of(3), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[3][1], batch_stage_kernel<3, 1, false>, bthreads_of(3), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[4][0], batch_stage_kernel<4, 0, false>, bthreads_of(4), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[4][1], batch_stage_kernel<4, 1, false>, bthreads_of(4), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[5][0], batch_stage_kernel<5, 0, false>, bthreads_of(5), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[5][1], batch_stage_kernel<5, 1, false>, bthreads_of(5), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[6][0], batch_stage_kernel<6, 0, false>, bthreads_of(6), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[6][1], batch_stage_kernel<6, 1, false>, bthreads_of(6), 0));
     max_ctas_per_sm = 1;
     for (int k = 2; k <= BATCH_KMAX; k++) {
         for (int ph = 0; ph < 2; ph++) {
@@ -497,6 +512,9 @@ int Batch::upload_tiles()
         d_counters = nc;
         counter_groups = ng;
     }
+    // every step leaves its counters zero for the next; their places move with
+    // the number of groups
+    if (d_counters) DGB_CUDA(cudaMemsetAsync(d_counters, 0, 3 * counter_groups * 2 * sizeof(int), stream));
     if ((int)tiles.size() > tile_capacity) {
         const int cap = std::max<int>((int)tiles.size(), 2 * tile_capacity);
         BatchTile* nt = nullptr;
@@ -524,17 +542,15 @@ int Batch::launch_step()
 {
     const int n = slot_hi;
     const int G = (int)groups.size();
-    DGB_CUDA(cudaMemsetAsync(d_counters, 0, 3 * G * 2 * sizeof(int), stream));
-    batch_step_begin<<<(n + 127) / 128, 128, 0, stream>>>(d_probs, n);
-    launches += 2;
-    // fork: group g runs its three stages on branch g % kBranches
-    const int nb = std::min(G, (int)kBranches);
-    DGB_CUDA(cudaEventRecord(fork_ev, stream));
+    // fork: group g runs its three stages on branch g % kBranches; one group
+    // alone stays on the main stream
+    const int nb = G > 1 ? std::min(G, (int)kBranches) : 0;
+    if (nb) DGB_CUDA(cudaEventRecord(fork_ev, stream));
     for (int b = 0; b < nb; b++) DGB_CUDA(cudaStreamWaitEvent(branch[b], fork_ev, 0));
     for (int g = 0; g < G; g++) {
         const Group& grp = groups[g];
         const int K = grp.K;
-        cudaStream_t bs = branch[g % kBranches];
+        cudaStream_t bs = nb ? branch[g % kBranches] : stream;
         for (int s = 0; s < 3; s++) {
             BatchArgs A;
             A.probs = d_probs;
@@ -548,17 +564,18 @@ int Batch::launch_step()
             for (int phase = 0; phase < 2; phase++) {
                 const int grid =
                     std::max(1, std::min(num_sms * std::min(ctas_per_sm, occ_k[K][phase]), A.n_tiles));
+                const bool after = s + phase > 0;
                 switch (K * 2 + phase) {
-                case 4: batch_stage_kernel<2, 0><<<grid, bthreads_of(2), 0, bs>>>(A, grp.ops); break;
-                case 5: batch_stage_kernel<2, 1><<<grid, bthreads_of(2), 0, bs>>>(A, grp.ops); break;
-                case 6: batch_stage_kernel<3, 0><<<grid, bthreads_of(3), 0, bs>>>(A, grp.ops); break;
-                case 7: batch_stage_kernel<3, 1><<<grid, bthreads_of(3), 0, bs>>>(A, grp.ops); break;
-                case 8: batch_stage_kernel<4, 0><<<grid, bthreads_of(4), 0, bs>>>(A, grp.ops); break;
-                case 9: batch_stage_kernel<4, 1><<<grid, bthreads_of(4), 0, bs>>>(A, grp.ops); break;
-                case 10: batch_stage_kernel<5, 0><<<grid, bthreads_of(5), 0, bs>>>(A, grp.ops); break;
-                case 11: batch_stage_kernel<5, 1><<<grid, bthreads_of(5), 0, bs>>>(A, grp.ops); break;
-                case 12: batch_stage_kernel<6, 0><<<grid, bthreads_of(6), 0, bs>>>(A, grp.ops); break;
-                case 13: batch_stage_kernel<6, 1><<<grid, bthreads_of(6), 0, bs>>>(A, grp.ops); break;
+                case 4: launch_batch<2, 0>(A, grp.ops, grid, after, bs); break;
+                case 5: launch_batch<2, 1>(A, grp.ops, grid, after, bs); break;
+                case 6: launch_batch<3, 0>(A, grp.ops, grid, after, bs); break;
+                case 7: launch_batch<3, 1>(A, grp.ops, grid, after, bs); break;
+                case 8: launch_batch<4, 0>(A, grp.ops, grid, after, bs); break;
+                case 9: launch_batch<4, 1>(A, grp.ops, grid, after, bs); break;
+                case 10: launch_batch<5, 0>(A, grp.ops, grid, after, bs); break;
+                case 11: launch_batch<5, 1>(A, grp.ops, grid, after, bs); break;
+                case 12: launch_batch<6, 0>(A, grp.ops, grid, after, bs); break;
+                case 13: launch_batch<6, 1>(A, grp.ops, grid, after, bs); break;
                 }
                 DGB_CUDA(cudaGetLastError());
                 launches++;
@@ -570,8 +587,10 @@ int Batch::launch_step()
         DGB_CUDA(cudaEventRecord(join_ev[b], branch[b]));
         DGB_CUDA(cudaStreamWaitEvent(stream, join_ev[b], 0));
     }
-    batch_step_end<<<(n + 127) / 128, 128, 0, stream>>>(d_probs, n);
+    const int nc = 3 * G * 2;
+    batch_step_end<<<(n + nc + 127) / 128, 128, 0, stream>>>(d_probs, n, d_counters, nc);
     DGB_CUDA(cudaGetLastError());
+    launches++;
     return DG_OK;
 }
 

@@ -7,8 +7,9 @@
 // so problems can join and leave (the serving form) without touching the
 // others.  Problems of one order that share one operator form a group; per
 // RK stage each group gets two launches of a persistent kernel of its order
-// (batch_stage_kernel<K>, K = N + 1 <= 6) that pull tiles (problem, first
-// element, element count) from an atomic counter: the LDG gradient of every
+// (batch_stage_kernel<K>, K = N + 1 <= 6) that take tiles (problem, first
+// element, element count), the first by block number, the rest from an atomic
+// counter: the LDG gradient of every
 // tile, then the stage update of every tile, with EPB(K) elements per pass of
 // a CTA of bthreads_of(K) threads; the number of passes per tile (tile size) is chosen per
 // order by the autotuner.  Groups run as parallel branches of the step.  The
@@ -44,11 +45,11 @@ __device__ __forceinline__ void batch_exterior(const BatchProblem& P, int face, 
     }
 }
 
-template <int K>
+template <int K, bool PDL>
 __device__ __forceinline__ float batch_in(const BatchProblem& P, const float* ub, const float* inc, int f, size_t off)
 {
-    float v = __ldg(ub + (size_t)f * P.fs + off);
-    if (inc) v += __ldg(inc + (size_t)f * P.fs + off);
+    float v = pdl_load<PDL>(ub + (size_t)f * P.fs + off);
+    if (inc) v += pdl_load<PDL>(inc + (size_t)f * P.fs + off);
     return v;
 }
 
@@ -131,7 +132,7 @@ struct BatchGradSmem {
 // to the buffer the pass before last read, which every owner finished before
 // the previous pass's barrier.  The owners' face-table codes of each pass
 // are loaded during the pass before.
-template <int K>
+template <int K, bool PDL>
 __device__ void batch_grad_tile(const BatchProblem& P, const BatchOps& ops, const BatchTile& T, int stage,
                                 unsigned char* smraw)
 {
@@ -155,14 +156,14 @@ __device__ void batch_grad_tile(const BatchProblem& P, const BatchOps& ops, cons
         batch_end_codes<K>(P, T, c0 + EPB, task, ls, a, code_next);
         // every other global load is issued before the first use
         float rho = 0.f;
-        if (act) rho = batch_in<K>(P, ub, inc, 0, (size_t)e * P.np + n);
+        if (act) rho = batch_in<K, PDL>(P, ub, inc, 0, (size_t)e * P.np + n);
         float ro[2] = {0.f, 0.f};
         if (owner) {
 #pragma unroll
             for (int side = 0; side < 2; side++) {
                 if (code[side] >= 0) {
                     const size_t o2 = (size_t)code[side] * P.np + b0 + (side ? 0 : (K - 1) * st);
-                    ro[side] = batch_in<K>(P, ub, inc, 0, o2);
+                    ro[side] = batch_in<K, PDL>(P, ub, inc, 0, o2);
                 } else {
                     float uo;
                     batch_exterior(P, -1 - code[side], stage, ro[side], uo);
@@ -192,7 +193,7 @@ __device__ void batch_grad_tile(const BatchProblem& P, const BatchOps& ops, cons
     }
 }
 
-template <int K>
+template <int K, bool PDL>
 __device__ void batch_stage_tile(const BatchProblem& P, const BatchOps& ops, const BatchTile& T, int stage,
                                  unsigned char* smraw)
 {
@@ -232,12 +233,12 @@ __device__ void batch_stage_tile(const BatchProblem& P, const BatchOps& ops, con
         if (act) {
 #pragma unroll
             for (int f = 0; f < 4; f++) {
-                ubv[f] = __ldg(ub + (size_t)f * P.fs + off);
-                if (inc) dv[f] = __ldg(inc + (size_t)f * P.fs + off);
+                ubv[f] = pdl_load<PDL>(ub + (size_t)f * P.fs + off);
+                if (inc) dv[f] = pdl_load<PDL>(inc + (size_t)f * P.fs + off);
                 if (final_stage) cmp[f] = P.comp[(size_t)f * P.fs + off];
             }
 #pragma unroll
-            for (int a = 0; a < 3; a++) q[a] = __ldg(P.q + (size_t)a * P.fs + off);
+            for (int a = 0; a < 3; a++) q[a] = pdl_load<PDL>(P.q + (size_t)a * P.fs + off);
         }
         float ro[R], uo[R], qo[R];
 #pragma unroll
@@ -248,9 +249,9 @@ __device__ void batch_stage_tile(const BatchProblem& P, const BatchOps& ops, con
             const FaceNodeArith<K> F(t);
             if (code[r] >= 0) {
                 const size_t o2 = (size_t)code[r] * P.np + F.nn;
-                ro[r] = batch_in<K>(P, ub, inc, 0, o2);
-                uo[r] = batch_in<K>(P, ub, inc, 1 + F.a, o2);
-                qo[r] = __ldg(P.q + (size_t)F.a * P.fs + o2);
+                ro[r] = batch_in<K, PDL>(P, ub, inc, 0, o2);
+                uo[r] = batch_in<K, PDL>(P, ub, inc, 1 + F.a, o2);
+                qo[r] = pdl_load<PDL>(P.q + (size_t)F.a * P.fs + o2);
             } else {
                 batch_exterior(P, -1 - code[r], stage, ro[r], uo[r]);
             }
@@ -407,46 +408,39 @@ __device__ __forceinline__ void load_problem(BatchProblem& dst, const BatchProbl
 // step without any kernel waiting on another's blocks, and separate kernels,
 // so that each gets its own register budget.  A persistent grid pulls the
 // group's tiles from an atomic counter.
-template <int K, int PHASE>
+template <int K, int PHASE, bool PDL>
 __global__ void __launch_bounds__(bthreads_of(K), batch_min_blocks(K, PHASE))
     batch_stage_kernel(BatchArgs A, const BatchOps ops)
 {
     __shared__ __align__(16) unsigned char smraw[batch_smem_bytes<K, PHASE>()];
     __shared__ BatchProblem P;
     __shared__ int tile_idx;
-    for (;;) {
-        if (threadIdx.x == 0) tile_idx = atomicAdd(A.counters + PHASE, 1);
-        __syncthreads();
-        const int ti = tile_idx;
-        if (ti >= A.n_tiles) break;
+    bool first = PDL;
+    // a block's first tile is its own number; the counter hands out the rest
+    for (int ti = blockIdx.x; ti < A.n_tiles;) {
         const BatchTile T = A.tiles[A.tile0 + ti];
         load_problem(P, A.probs + T.prob);
-        __syncthreads();
-        if (P.active) {
-            if constexpr (PHASE == 0) batch_grad_tile<K>(P, ops, T, A.stage, smraw);
-            else batch_stage_tile<K>(P, ops, T, A.stage, smraw);
+        if (first) {
+            // tiles, counters and descriptors are the same for all kernels of a step
+            pdl_wait();
+            pdl_next();
+            first = false;
         }
         __syncthreads();
+        if (P.active) {
+            if constexpr (PHASE == 0) batch_grad_tile<K, PDL>(P, ops, T, A.stage, smraw);
+            else batch_stage_tile<K, PDL>(P, ops, T, A.stage, smraw);
+        }
+        if (A.n_tiles <= gridDim.x) break;
+        if (threadIdx.x == 0) tile_idx = gridDim.x + atomicAdd(A.counters + PHASE, 1);
+        __syncthreads();
+        ti = tile_idx;
     }
 }
 
-// Writes one problem descriptor into its slot.  The descriptor travels as a
-// kernel argument (copied at launch), so the host needs no page-locked
-// staging and no synchronisation to add or retire a problem.
-__global__ void batch_set_problem(BatchProblem* __restrict__ dst, const BatchProblem P)
+// Source pressures at the stage times of a problem's next step.
+__device__ __forceinline__ void batch_source(BatchProblem& P)
 {
-    const int* s = reinterpret_cast<const int*>(&P);
-    int* d = reinterpret_cast<int*>(dst);
-    for (int i = threadIdx.x; i < (int)(sizeof(BatchProblem) / sizeof(int)); i += blockDim.x) d[i] = s[i];
-}
-
-// Per-problem bookkeeping around a step (one thread per problem).
-__global__ void batch_step_begin(BatchProblem* probs, int n)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    BatchProblem& P = probs[i];
-    if (!P.active) return;
     const double ts[3] = {P.t, P.t + P.dt, P.t + 0.5 * P.dt};
     for (int s = 0; s < 3; s++) {
         double p = 0.0;
@@ -458,16 +452,35 @@ __global__ void batch_step_begin(BatchProblem* probs, int n)
     }
 }
 
-__global__ void batch_step_end(BatchProblem* probs, int n)
+// Writes one problem descriptor into its slot, with the source pressures of
+// its next step.  The descriptor travels as a kernel argument (copied at
+// launch), so the host needs no page-locked staging and no synchronisation to
+// add or retire a problem.
+__global__ void batch_set_problem(BatchProblem* __restrict__ dst, const BatchProblem P)
+{
+    const int* s = reinterpret_cast<const int*>(&P);
+    int* d = reinterpret_cast<int*>(dst);
+    for (int i = threadIdx.x; i < (int)(sizeof(BatchProblem) / sizeof(int)); i += blockDim.x) d[i] = s[i];
+    __syncthreads();
+    if (threadIdx.x == 0 && dst->active) batch_source(*dst);
+}
+
+// Bookkeeping after a step, which also prepares the next one (one thread per
+// problem, then per tile counter): a step is its stages and this launch.
+__global__ void batch_step_end(BatchProblem* probs, int n, int* counters, int n_counters)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= n) {
+        if (i - n < n_counters) counters[i - n] = 0;
+        return;
+    }
     BatchProblem& P = probs[i];
     if (!P.active) return;
     P.t += P.dt;
     P.cur ^= 1;
     P.steps_done++;
     if (--P.steps_left <= 0) P.active = 0;
+    batch_source(P);
 }
 
 }  // namespace dg

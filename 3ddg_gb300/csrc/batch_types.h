@@ -50,7 +50,7 @@ struct BatchArgs {
     BatchProblem* probs;
     const BatchTile* tiles;
     int tile0, n_tiles;    // this launch's tiles: tiles[tile0 .. tile0 + n_tiles)
-    int* counters;         // [2]: phase-1 and phase-2 tile counters, zeroed before the launch
+    int* counters;         // [2]: tiles taken beyond each block's first, per phase; zero at the launch
     int stage;
 };
 

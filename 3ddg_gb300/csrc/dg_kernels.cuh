@@ -50,6 +50,8 @@
 #include <cstddef>
 #include <cstdint>
 
+#include "pdl.cuh"
+
 namespace dg {
 
 __host__ __device__ constexpr int npt_of(int K) { return (K * K * K + 31) / 32 * 32; }
@@ -223,11 +225,11 @@ struct GradSmem {
     T fl[3][2][K * K];
 };
 
-template <bool INCR, typename T>
+template <bool INCR, bool PDL = false, typename T>
 __device__ __forceinline__ T load_in(const StageIO<T>& io, int f, size_t off)
 {
-    T v = __ldg(io.src + (size_t)f * io.fs + off);
-    if (INCR && io.inc) v += __ldg(io.inc + (size_t)f * io.fs + off);
+    T v = pdl_load<PDL>(io.src + (size_t)f * io.fs + off);
+    if (INCR && io.inc) v += pdl_load<PDL>(io.inc + (size_t)f * io.fs + off);
     return v;
 }
 
@@ -419,13 +421,21 @@ __device__ __forceinline__ void grad_line_faces(const OpConst<T, K>& Cv, const S
     }
 }
 
+// Face-table entries of the two ends of a line along axis a.
+template <typename T>
+__device__ __forceinline__ void line_end_codes(const MeshDev<T>& m, int e, int a, int code[2])
+{
+#pragma unroll
+    for (int side = 0; side < 2; side++) code[side] = __ldg(m.nbr + (size_t)e * 6 + 2 * a + side);
+}
+
 // Neighbour (or exterior) values of the two face nodes at the ends of line t
 // along axis a, for the line owners above: drho always, the normal velocity
 // with WITH_U, the gradient with WITH_Q (arrays not asked for are zeroed).
-template <bool INCR, bool WITH_U, bool WITH_Q, typename T, int K>
+template <bool INCR, bool WITH_U, bool WITH_Q, bool PDL, typename T, int K>
 __device__ __forceinline__ void line_end_values(const StageIO<T>& io, const MeshDev<T>& m,
-                                                const OpConst<T, K>& C, int e, int a, int t, T ro[2], T uo[2],
-                                                T qo[2])
+                                                const OpConst<T, K>& C, const int codes[2], int a, int t, T ro[2],
+                                                T uo[2], T qo[2])
 {
     const int st = axis_stride<K>(a);
     const int b0 = a == 0 ? t : (a == 1 ? (t % K) * K * K + t / K : t * K);
@@ -434,12 +444,12 @@ __device__ __forceinline__ void line_end_values(const StageIO<T>& io, const Mesh
         ro[side] = T(0);
         uo[side] = T(0);
         qo[side] = T(0);
-        const int code = __ldg(m.nbr + (size_t)e * 6 + 2 * a + side);
+        const int code = codes[side];
         if (code >= 0) {
             const size_t o2 = (size_t)code * io.np + b0 + (side ? 0 : (K - 1) * st);
-            ro[side] = load_in<INCR>(io, 0, o2);
-            if (WITH_U) uo[side] = load_in<INCR>(io, 1 + a, o2);
-            if (WITH_Q) qo[side] = __ldg(io.q + (size_t)a * io.fs + o2);
+            ro[side] = load_in<INCR, PDL>(io, 0, o2);
+            if (WITH_U) uo[side] = load_in<INCR, PDL>(io, 1 + a, o2);
+            if (WITH_Q) qo[side] = pdl_load<PDL>(io.q + (size_t)a * io.fs + o2);
         } else {
             T u2;
             exterior<T, K>(m, C, -1 - code, side, t, ro[side], u2);
@@ -457,7 +467,7 @@ __host__ __device__ constexpr int grad_min_blocks()
     return (sizeof(T) == 4 && K <= 5) ? 65536 / (40 * npt_of(K) * epb_of(K)) : 0;
 }
 
-template <typename T, int K, bool INCR>
+template <typename T, int K, bool INCR, bool PDL>
 __global__ void __launch_bounds__(npt_of(K) * epb_of(K), (grad_min_blocks<T, K>()))
 ldg_gradient_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__ Cp, const OpConst<T, K> Cv)
 {
@@ -479,9 +489,15 @@ ldg_gradient_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict
         constexpr int WPA = (K2 + 31) / 32;
         const int w = n / 32, a = w / WPA, t = (w % WPA) * 32 + n % 32;
         const bool owner = live && a < 3 && t < K2;
+        int code[2] = {0, 0};
+        if (owner) line_end_codes(m, e, a, code);
+        if constexpr (PDL) {
+            pdl_wait();
+            pdl_next();
+        }
         T rho = T(0), ro[2] = {T(0), T(0)}, unused_u[2], unused_q[2];
-        if (act) rho = load_in<INCR>(io, 0, (size_t)e * io.np + n);
-        if (owner) line_end_values<INCR, false, false, T, K>(io, m, C, e, a, t, ro, unused_u, unused_q);
+        if (act) rho = load_in<INCR, PDL>(io, 0, (size_t)e * io.np + n);
+        if (owner) line_end_values<INCR, false, false, PDL, T, K>(io, m, C, code, a, t, ro, unused_u, unused_q);
         S.r[n] = rho;
         __syncthreads();
         if (owner) {
@@ -503,8 +519,12 @@ ldg_gradient_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict
                 code[r] = __ldg(m.nbr + (size_t)e * 6 + 2 * F.a + F.side);
             }
         }
+        if constexpr (PDL) {
+            pdl_wait();
+            pdl_next();
+        }
         T rho = T(0);
-        if (act) rho = load_in<INCR>(io, 0, (size_t)e * io.np + n);
+        if (act) rho = load_in<INCR, PDL>(io, 0, (size_t)e * io.np + n);
         T ro[R];
 #pragma unroll
         for (int r = 0; r < R; r++) {
@@ -513,7 +533,7 @@ ldg_gradient_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict
             if (!live || t >= NF) continue;
             const FaceNode<K> F(t);
             if (code[r] >= 0) {
-                ro[r] = load_in<INCR>(io, 0, (size_t)code[r] * io.np + F.nn);
+                ro[r] = load_in<INCR, PDL>(io, 0, (size_t)code[r] * io.np + F.nn);
             } else {
                 T uo;
                 exterior<T, K>(m, C, -1 - code[r], F.side, F.fi, ro[r], uo);
@@ -777,7 +797,7 @@ __host__ __device__ constexpr int incr_min_blocks()
     return (sizeof(T) == 4 && K == 5) ? 12 : 0;
 }
 
-template <typename T, int K, bool DIFF>
+template <typename T, int K, bool DIFF, bool PDL>
 __global__ void __launch_bounds__(npt_of(K) * epb_of(K), (incr_min_blocks<T, K>()))
 incr_stage_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__ Cp, const OpConst<T, K> Cv,
                   int do_adv, int do_sponge)
@@ -798,8 +818,10 @@ incr_stage_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__
     const int la = n / 32 / WPA, lt = (n / 32 % WPA) * 32 + n % 32;
     const bool owner = LINES && live && la < 3 && lt < K2;
 
-    int code[R];
-    if constexpr (!LINES) {
+    int code[R > 2 ? R : 2] = {0, 0};
+    if constexpr (LINES) {
+        if (owner) line_end_codes(m, e, la, code);
+    } else {
 #pragma unroll
         for (int r = 0; r < R; r++) {
             const int t = n + r * NPT;
@@ -811,24 +833,28 @@ incr_stage_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__
         }
     }
     const T sig = (act && do_sponge) ? __ldg(m.sigma + e) : T(0);
+    if constexpr (PDL) {
+        pdl_wait();
+        pdl_next();
+    }
     T ub[4] = {T(0), T(0), T(0), T(0)}, dv[4] = {T(0), T(0), T(0), T(0)};
     T cmp[4] = {T(0), T(0), T(0), T(0)}, q[3] = {T(0), T(0), T(0)};
     if (act) {
 #pragma unroll
         for (int f = 0; f < 4; f++) {
-            ub[f] = __ldg(io.src + (size_t)f * io.fs + off);
-            if (io.inc) dv[f] = __ldg(io.inc + (size_t)f * io.fs + off);
+            ub[f] = pdl_load<PDL>(io.src + (size_t)f * io.fs + off);
+            if (io.inc) dv[f] = pdl_load<PDL>(io.inc + (size_t)f * io.fs + off);
             if (io.final_stage) cmp[f] = io.comp[(size_t)f * io.fs + off];
         }
         if (DIFF)
 #pragma unroll
-            for (int a = 0; a < 3; a++) q[a] = __ldg(io.q + (size_t)a * io.fs + off);
+            for (int a = 0; a < 3; a++) q[a] = pdl_load<PDL>(io.q + (size_t)a * io.fs + off);
     }
     // Neighbour (or exterior) values: of the two ends of the owned line
     // (LINES), else of the densely assigned face nodes.
     T ro[R > 2 ? R : 2], uo[R > 2 ? R : 2], qo[R > 2 ? R : 2];
     if constexpr (LINES) {
-        if (owner) line_end_values<true, true, DIFF, T, K>(io, m, C, e, la, lt, ro, uo, qo);
+        if (owner) line_end_values<true, true, DIFF, PDL, T, K>(io, m, C, code, la, lt, ro, uo, qo);
     } else {
 #pragma unroll
         for (int r = 0; r < R; r++) {
@@ -838,9 +864,9 @@ incr_stage_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__
             const FaceNode<K> F(t);
             if (code[r] >= 0) {
                 const size_t o2 = (size_t)code[r] * io.np + F.nn;
-                ro[r] = load_in<true>(io, 0, o2);
-                uo[r] = load_in<true>(io, 1 + F.a, o2);
-                if (DIFF) qo[r] = __ldg(io.q + (size_t)F.a * io.fs + o2);
+                ro[r] = load_in<true, PDL>(io, 0, o2);
+                uo[r] = load_in<true, PDL>(io, 1 + F.a, o2);
+                if (DIFF) qo[r] = pdl_load<PDL>(io.q + (size_t)F.a * io.fs + o2);
             } else {
                 exterior<T, K>(m, C, -1 - code[r], F.side, F.fi, ro[r], uo[r]);
             }

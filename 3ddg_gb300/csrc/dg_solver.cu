@@ -161,14 +161,18 @@ void launch_grad(Solver& s, const StageIO<T>& io, const MeshDev<T>& md)
     bool done = false;
     if constexpr (!INCR && sizeof(T) == 8) {
         if (s.fix_ok[3]) {
-            ldg_gradient_fix_kernel<K><<<(md.n_elem + fix_epb(K) - 1) / fix_epb(K), fix_threads(K), 0, s.stream>>>(
-                io, md, host_const<T, K>(s, 3), fix_set<K>(s).grad);
+            launch_pdl(ldg_gradient_fix_kernel<K>, (md.n_elem + fix_epb(K) - 1) / fix_epb(K), fix_threads(K), s.stream,
+                       io, md, host_const<T, K>(s, 3), fix_set<K>(s).grad);
             done = true;
         }
     }
     if (!done)
-        ldg_gradient_kernel<T, K, INCR><<<grid, block, 0, s.stream>>>(io, md, const_ptr<T, K>(s, 3),
-                                                                        host_const<T, K>(s, 3));
+        if (s.short_launches())
+            launch_pdl(ldg_gradient_kernel<T, K, INCR, true>, grid, block, s.stream, io, md, const_ptr<T, K>(s, 3),
+                       host_const<T, K>(s, 3));
+        else
+            ldg_gradient_kernel<T, K, INCR, false><<<grid, block, 0, s.stream>>>(io, md, const_ptr<T, K>(s, 3),
+                                                                                host_const<T, K>(s, 3));
     s.prof_end(1, ev, grad_bytes(s, io), grad_flops(s));
     s.launches++;
 }
@@ -180,9 +184,9 @@ template <int K, bool DIFF, int FLUX, bool PACK = false>
 void launch_plain_mode(const Solver& s, int slot, const StageIO<double>& io, const MeshDev<double>& md)
 {
     if (s.fix_ok[slot])
-        stage_fix_kernel<K, DIFF, FLUX, PACK>
-            <<<(md.n_elem + fix_epb(K) - 1) / fix_epb(K), fix_threads(K), 0, s.stream>>>(
-                io, md, host_const<double, K>(s, slot), fix_set<K>(s).stage[slot], s.p.eval_advect, s.p.eval_sponge);
+        launch_pdl(stage_fix_kernel<K, DIFF, FLUX, PACK>, (md.n_elem + fix_epb(K) - 1) / fix_epb(K), fix_threads(K),
+                   s.stream, io, md, host_const<double, K>(s, slot), fix_set<K>(s).stage[slot], s.p.eval_advect,
+                   s.p.eval_sponge);
     else
         stage_kernel<double, K, DIFF, FLUX>
             <<<(md.n_elem + epb_of(K) - 1) / epb_of(K), dim3(npt_of(K), epb_of(K)), 0, s.stream>>>(
@@ -205,6 +209,18 @@ void launch_plain(const Solver& s, int slot, const StageIO<double>& io, const Me
     }
 }
 
+template <typename T, int K, bool DIFF>
+void launch_incr(const Solver& s, dim3 grid, dim3 block, const StageIO<T>& io, const MeshDev<T>& md,
+                 const OpConst<T, K>* Cp, const OpConst<T, K>& Cv)
+{
+    if (s.short_launches())
+        launch_pdl(incr_stage_kernel<T, K, DIFF, true>, grid, block, s.stream, io, md, Cp, Cv, s.p.eval_advect,
+                   s.p.eval_sponge);
+    else
+        incr_stage_kernel<T, K, DIFF, false><<<grid, block, 0, s.stream>>>(io, md, Cp, Cv, s.p.eval_advect,
+                                                                           s.p.eval_sponge);
+}
+
 template <typename T, int K, bool INCR>
 void launch_stage(Solver& s, const StageIO<T>& io, const MeshDev<T>& md, int slot)
 {
@@ -215,12 +231,8 @@ void launch_stage(Solver& s, const StageIO<T>& io, const MeshDev<T>& md, int slo
         const dim3 block(npt_of(K), epb_of(K));
         const dim3 grid((md.n_elem + epb_of(K) - 1) / epb_of(K));
         const OpConst<T, K>& Cv = host_const<T, K>(s, slot);
-        if (s.p.eval_diff)
-            incr_stage_kernel<T, K, true><<<grid, block, 0, s.stream>>>(io, md, Cp, Cv, s.p.eval_advect,
-                                                                       s.p.eval_sponge);
-        else
-            incr_stage_kernel<T, K, false><<<grid, block, 0, s.stream>>>(io, md, Cp, Cv, s.p.eval_advect,
-                                                                        s.p.eval_sponge);
+        if (s.p.eval_diff) launch_incr<T, K, true>(s, grid, block, io, md, Cp, Cv);
+        else launch_incr<T, K, false>(s, grid, block, io, md, Cp, Cv);
     } else {
         if (s.p.eval_diff) launch_plain<K, true>(s, slot, io, md);
         else launch_plain<K, false>(s, slot, io, md);

@@ -12,6 +12,7 @@
 
 #include "dg_kernels.cuh"
 #include "fixed_line.cuh"
+#include "pdl.cuh"
 
 namespace dg {
 
@@ -67,29 +68,42 @@ struct FixTask {
     }
 };
 
-// Neighbour (or exterior) values at the two ends of a line of element e: drho
+// Face-table entries of the two ends of this thread's lines.
+template <int K>
+__device__ __forceinline__ void fix_codes(const MeshDev<double>& m, int e0, int (&code)[fix_rounds(K)][2])
+{
+#pragma unroll
+    for (int r = 0; r < fix_rounds(K); r++) {
+        const int task = threadIdx.x + r * fix_threads(K);
+        const FixTask<K> L(task);
+        const bool live = task < fix_epb(K) * 3 * K * K && e0 + L.le < m.n_elem;
+#pragma unroll
+        for (int s = 0; s < 2; s++) code[r][s] = live ? __ldg(m.nbr + (size_t)(e0 + L.le) * 6 + 2 * L.a + s) : 0;
+    }
+}
+
+// Neighbour (or exterior) values at the two ends of a line: drho
 // alone, or (FLUXES) the momentum and mass fluxes f0, f1 and with WITH_Q the
 // gradient qo, read from flux_in in flux mode 2 and else evaluated.
 template <bool FLUXES, bool WITH_Q, int K, int FLUX = 0>
 __device__ __forceinline__ void fix_end_values(const StageIO<double>& io, const MeshDev<double>& m,
-                                               const OpConst<double, K>& C, int e, const FixTask<K>& L,
-                                               double (&f0)[2], double (&f1)[2], double (&qo)[2])
+                                               const OpConst<double, K>& C, const int (&code)[2],
+                                               const FixTask<K>& L, double (&f0)[2], double (&f1)[2], double (&qo)[2])
 {
-    const int code[2] = {__ldg(m.nbr + (size_t)e * 6 + 2 * L.a), __ldg(m.nbr + (size_t)e * 6 + 2 * L.a + 1)};
 #pragma unroll
     for (int side = 0; side < 2; side++) {
         f1[side] = qo[side] = 0.0;
         double ro, uo = 0.0;
         if (code[side] >= 0) {
             const size_t o2 = (size_t)code[side] * io.np + L.b0 + (side ? 0 : (K - 1) * L.st);
-            if (WITH_Q) qo[side] = __ldg(io.q + (size_t)L.a * io.fs + o2);
+            if (WITH_Q) qo[side] = io.q[(size_t)L.a * io.fs + o2];
             if (FLUXES && FLUX == 2) {
-                f0[side] = __ldg(io.flux_in + o2);
-                f1[side] = __ldg(io.flux_in + (size_t)(1 + L.a) * io.fs + o2);
+                f0[side] = io.flux_in[o2];
+                f1[side] = io.flux_in[(size_t)(1 + L.a) * io.fs + o2];
                 continue;
             }
-            ro = __ldg(io.src + o2);
-            if (FLUXES) uo = __ldg(io.src + (size_t)(1 + L.a) * io.fs + o2);
+            ro = io.src[o2];
+            if (FLUXES) uo = io.src[(size_t)(1 + L.a) * io.fs + o2];
         } else if (m.bnd_src) {
             exterior<double, K>(m, C, -1 - code[side], side, L.fi, ro, uo);
         } else {
@@ -148,6 +162,10 @@ ldg_gradient_fix_kernel(StageIO<double> io, MeshDev<double> m, const __grid_cons
     const int el = tid / K3, n = tid - el * K3;
     const bool act = el < EPB && e0 + el < m.n_elem;
     const size_t off = (size_t)(e0 + el) * io.np + n;
+    int code[RL][2];
+    fix_codes<K>(m, e0, code);
+    pdl_wait();
+    pdl_next();
     if (act) copy_async8(&sm[el].r[fix_slot<K>(n)], io.src + off);
     copy_async_commit();
     double ro[RL][2];
@@ -158,7 +176,7 @@ ldg_gradient_fix_kernel(StageIO<double> io, MeshDev<double> m, const __grid_cons
         const FixTask<K> L(task);
         if (task >= EPB * 3 * K2 || e0 + L.le >= m.n_elem) continue;
         double unused_u[2], unused_q[2];
-        fix_end_values<false, false, K>(io, m, C, e0 + L.le, L, ro[r], unused_u, unused_q);
+        fix_end_values<false, false, K>(io, m, C, code[r], L, ro[r], unused_u, unused_q);
     }
     copy_async_wait<0>();
     __syncthreads();
@@ -355,6 +373,10 @@ stage_fix_kernel(StageIO<double> io, MeshDev<double> m, const __grid_constant__ 
     const int e = e0 + el;
     const bool act = el < EPB && e < m.n_elem;
     const size_t off = (size_t)e * io.np + n;
+    int code[RL][2];
+    fix_codes<K>(m, e0, code);
+    pdl_wait();
+    pdl_next();
 
     double s4[4] = {0.0, 0.0, 0.0, 0.0};
     if (act) {
@@ -379,7 +401,7 @@ stage_fix_kernel(StageIO<double> io, MeshDev<double> m, const __grid_constant__ 
         copy_async_commit();
         if (FLUX != 2) {
 #pragma unroll
-            for (int f = 0; f < 4; f++) s4[f] = __ldg(io.src + (size_t)f * io.fs + off);
+            for (int f = 0; f < 4; f++) s4[f] = io.src[(size_t)f * io.fs + off];
             S.fm[sn] = do_adv ? momentum_flux(s4[0], C.k1, C.k2) : 0.0;
 #pragma unroll
             for (int a = 0; a < 3; a++)
@@ -395,7 +417,7 @@ stage_fix_kernel(StageIO<double> io, MeshDev<double> m, const __grid_constant__ 
         const int task = tid + r * T;
         const FixTask<K> L(task);
         if (task >= EPB * 3 * K2 || e0 + L.le >= m.n_elem) continue;
-        fix_end_values<true, DIFF, K, FLUX>(io, m, C, e0 + L.le, L, fmo[r], fao[r], qo[r]);
+        fix_end_values<true, DIFF, K, FLUX>(io, m, C, code[r], L, fmo[r], fao[r], qo[r]);
         if (FLUX != 2 && !do_adv) fmo[r][0] = fmo[r][1] = fao[r][0] = fao[r][1] = 0.0;
     }
     copy_async_wait<1>();
@@ -432,7 +454,7 @@ stage_fix_kernel(StageIO<double> io, MeshDev<double> m, const __grid_constant__ 
 #pragma unroll
     for (int f = 0; f < 4; f++) {
         const size_t o = (size_t)f * io.fs + off;
-        if (FLUX == 2) s4[f] = STAGED ? st[f][tid] : __ldg(io.src + o);
+        if (FLUX == 2) s4[f] = STAGED ? st[f][tid] : io.src[o];
         double v = rr[f] + s4[f] * cbe;
         if (io.old) v += (STAGED ? st[4 + f][tid] : io.old[o]) * io.cc;
         io.dst[o] = v;

@@ -83,6 +83,14 @@ struct Solver {
 
     bool fp64() const { return p.precision == DG_PRECISION_FP64; }
     size_t gsize() const { return (size_t)mesh.n_elem * mesh.K * mesh.K * mesh.K; }
+    // FP32 launches of up to about 20 us start under the one before
+    // (launch_pdl): 8^3 elements at N = 3, 656 -> 422 us per 120 launches.  Above,
+    // the dependent form's plain loads and early wait cost more than the gap
+    // (64^3 at N = 4: 17.4 -> 19.4 ms per 48 launches; 13,800 elements at N = 3,
+    // 0.88 M nodes: 1.558 -> 1.570 ms per 120).  The FP64 kernels are always
+    // launched so: 8^3 at N = 3, 797 -> 553 us per 120; 64^3 at N = 4, 15.9 ->
+    // 15.3 ms per 18.
+    bool short_launches() const { return gsize() <= 800000; }
     size_t device_bytes() const;
     void* state_ptr() const;
 
