@@ -1,18 +1,20 @@
 // sm_103a kernels for one stage of the DG right-hand side and its RK update.
 //
 // Two launches per RK stage (one without diffusion):
-//   ldg_gradient_kernel (FP32), ldg_gradient_fix_kernel (FP64, fix_kernels.cuh)
+//   ldg_gradient_fix_kernel (FP64, fix_kernels.cuh), incr_gradient_kernel
+//   (FP32, incr_kernels.cuh)
 //                        G_a = -D_c d(drho)/dx_a by LDG with the central flux
 //                        (Element::OperateQFromDRho, cppsrc/Element.cpp:623-690;
 //                        stored pre-multiplied by -D_c, the diffusive flux)
-//   stage_fix_kernel (FP64, fix_kernels.cuh), incr_stage_kernel (FP32
-//                        increment form)
+//   stage_fix_kernel (FP64), incr_stage_kernel (FP32 increment form)
 //                        volume + face terms of the advection operator
 //                        (Element::OperateUFromV, cppsrc/Element.cpp:475-620),
 //                        LDG divergence (Element::OperateDRhoFromQ, :691-758),
 //                        sponge (Element::OperateSponge, :760-781) and the RK
 //                        stage combination (Element::selfWeightedAdd, :288-307)
 //                        fused into one pass over the state.
+// This file: what they share, and the FP64 kernels for operators without a
+// fixed-point form (ldg_gradient_kernel, stage_kernel).
 //
 // Mapping: one thread per node, one warp-aligned slice of NPT threads per
 // element, EPB elements per CTA.  Each thread loads its node (and the
@@ -35,11 +37,6 @@
 // centro-antisymmetric).  Each stage writes the volume fluxes of its output
 // for the next stage to read (flux modes), so no face neighbour's flux is
 // evaluated twice.
-//
-// FP32 (bound by the L1 data pipe, load latency and issue): for K >= 5 line
-// owners (a warp per axis, a lane per line) evaluate their line's two face
-// terms and its K outputs with the operator as kernel parameters, instead of
-// every node summing its own three lines from shared memory.
 //
 // Neighbour face values are read straight from the neighbour element (same
 // block or another block of the same HBM pool) through the face table, which
@@ -225,12 +222,10 @@ struct GradSmem {
     T fl[3][2][K * K];
 };
 
-template <bool INCR, bool PDL = false, typename T>
+template <typename T>
 __device__ __forceinline__ T load_in(const StageIO<T>& io, int f, size_t off)
 {
-    T v = pdl_load<PDL>(io.src + (size_t)f * io.fs + off);
-    if (INCR && io.inc) v += pdl_load<PDL>(io.inc + (size_t)f * io.fs + off);
-    return v;
+    return __ldg(io.src + (size_t)f * io.fs + off);
 }
 
 // Exterior value at a domain-boundary face node: the tone burst on the source
@@ -342,139 +337,11 @@ struct OpRows {
     }
 };
 
-// First node of line t along axis A (lines numbered like the face nodes fi),
-// for the line owners below.
-template <int A, int K>
-__device__ __forceinline__ int line_base(int t)
-{
-    return A == 0 ? t : (A == 1 ? (t % K) * K * K + t / K : t * K);
-}
-
-// Line owner with its own face terms (FP32, K >= 5): the two ends of line t
-// along axis A are the face nodes (A, 0, t) and (A, 1, t), so the owner
-// evaluates both numerical fluxes itself (neighbour values ro/uo/qo[side],
-// prefetched; own values from shared memory) and then the line sums.  The
-// face coefficients come from kernel parameters with a compile-time axis.
-template <int A, bool DIFF, typename T, int K, typename Smem>
-__device__ __forceinline__ void stage_line_faces(const OpConst<T, K>& Cv, Smem& S, int t, const T ro[2],
-                                                 const T uo[2], const T qo[2], int do_adv)
-{
-    constexpr int st = axis_stride<K>(A);
-    const int b0 = line_base<A, K>(t);
-    typename Pair<T>::type g[2];
-#pragma unroll
-    for (int side = 0; side < 2; side++) {
-        const int nf = b0 + (side ? (K - 1) * st : 0);
-        const T fm_s = S.f[A][nf].x, fa_s = S.m[A][nf];
-        T gm = T(0), gr = T(0);
-        if (do_adv) {
-            const T fmo = momentum_flux(ro[side], Cv.k1, Cv.k2);
-            const T fao = mass_flux(uo[side], ro[side], Cv.r0, Cv.linear_mass);
-            const T* cm = Cv.cM[A][side];
-            const T* cr = Cv.cA[A][side];
-            gm = fmo * cm[0] + fm_s * cm[1] + fao * cm[2] + fa_s * cm[3];
-            gr = fmo * cr[0] + fm_s * cr[1] + fao * cr[2] + fa_s * cr[3];
-        }
-        if (DIFF) gr += Cv.cQ[A][side] * (qo[side] + S.q[A][nf]);
-        g[side].x = gm;
-        g[side].y = gr;
-    }
-    typename Pair<T>::type v[K];
-#pragma unroll
-    for (int j = 0; j < K; j++) v[j] = S.f[A][b0 + j * st];
-#pragma unroll
-    for (int i = 0; i < K; i++) {
-        const T* row = Cv.rows[A][i];
-        T sm = row[K] * g[0].x, sr = row[K] * g[0].y;
-        sm += row[K + 1] * g[1].x;
-        sr += row[K + 1] * g[1].y;
-#pragma unroll
-        for (int j = 0; j < K; j++) {
-            sm += row[j] * v[j].x;
-            sr += row[j] * v[j].y;
-        }
-        S.m[A][b0 + i * st] = sr;
-        S.q[A][b0 + i * st] = sm;
-    }
-}
-
-// The same for the LDG gradient: central flux of drho at both ends; the
-// owner stores its line's K values of G_A at q_elem (the element's G_A).
-template <int A, typename T, int K, typename Smem>
-__device__ __forceinline__ void grad_line_faces(const OpConst<T, K>& Cv, const Smem& S, int t, const T ro[2],
-                                                T* __restrict__ q_elem)
-{
-    constexpr int st = axis_stride<K>(A);
-    const int b0 = line_base<A, K>(t);
-    T v[K];
-#pragma unroll
-    for (int j = 0; j < K; j++) v[j] = S.r[b0 + j * st];
-    const T f0 = ro[0] + v[0], fN = ro[1] + v[K - 1];  // flux factors are in the lift columns
-#pragma unroll
-    for (int i = 0; i < K; i++) {
-        const T* row = Cv.rows[A][i];
-        T s2 = row[K] * f0;
-        s2 += row[K + 1] * fN;
-#pragma unroll
-        for (int j = 0; j < K; j++) s2 += row[j] * v[j];
-        q_elem[b0 + i * st] = s2;
-    }
-}
-
-// Face-table entries of the two ends of a line along axis a.
-template <typename T>
-__device__ __forceinline__ void line_end_codes(const MeshDev<T>& m, int e, int a, int code[2])
-{
-#pragma unroll
-    for (int side = 0; side < 2; side++) code[side] = __ldg(m.nbr + (size_t)e * 6 + 2 * a + side);
-}
-
-// Neighbour (or exterior) values of the two face nodes at the ends of line t
-// along axis a, for the line owners above: drho always, the normal velocity
-// with WITH_U, the gradient with WITH_Q (arrays not asked for are zeroed).
-template <bool INCR, bool WITH_U, bool WITH_Q, bool PDL, typename T, int K>
-__device__ __forceinline__ void line_end_values(const StageIO<T>& io, const MeshDev<T>& m,
-                                                const OpConst<T, K>& C, const int codes[2], int a, int t, T ro[2],
-                                                T uo[2], T qo[2])
-{
-    const int st = axis_stride<K>(a);
-    const int b0 = a == 0 ? t : (a == 1 ? (t % K) * K * K + t / K : t * K);
-#pragma unroll
-    for (int side = 0; side < 2; side++) {
-        ro[side] = T(0);
-        uo[side] = T(0);
-        qo[side] = T(0);
-        const int code = codes[side];
-        if (code >= 0) {
-            const size_t o2 = (size_t)code * io.np + b0 + (side ? 0 : (K - 1) * st);
-            ro[side] = load_in<INCR, PDL>(io, 0, o2);
-            if (WITH_U) uo[side] = load_in<INCR, PDL>(io, 1 + a, o2);
-            if (WITH_Q) qo[side] = pdl_load<PDL>(io.q + (size_t)a * io.fs + o2);
-        } else {
-            T u2;
-            exterior<T, K>(m, C, -1 - code, side, t, ro[side], u2);
-            if (WITH_U) uo[side] = u2;
-        }
-    }
-}
-
-// Resident CTAs per SM asked of the compiler for the gradient kernel (0: no
-// request): the FP32 kernel waits on memory latency and fits in 40 registers
-// without spilling up to K = 5.
 template <typename T, int K>
-__host__ __device__ constexpr int grad_min_blocks()
-{
-    return (sizeof(T) == 4 && K <= 5) ? 65536 / (40 * npt_of(K) * epb_of(K)) : 0;
-}
-
-template <typename T, int K, bool INCR, bool PDL>
-__global__ void __launch_bounds__(npt_of(K) * epb_of(K), (grad_min_blocks<T, K>()))
-ldg_gradient_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__ Cp, const OpConst<T, K> Cv)
+__global__ void __launch_bounds__(npt_of(K) * epb_of(K))
+ldg_gradient_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__ Cp)
 {
     constexpr int K2 = K * K, K3 = K * K * K, NPT = npt_of(K), NF = 6 * K2, R = (NF + NPT - 1) / NPT;
-    // FP32 (bound by the L1 data pipe) with K >= 5: line owners, as in
-    // incr_stage_kernel; FP64 (bound by the FP64 pipe) keeps per-node sums.
-    constexpr bool LINES = INCR && K >= 5;
     __shared__ GradSmem<T, K> sm_all[epb_of(K)];
     GradSmem<T, K>& S = sm_all[threadIdx.y];
     const OpConst<T, K>& C = *Cp;
@@ -483,86 +350,57 @@ ldg_gradient_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict
     const bool live = e < m.n_elem;
     const bool act = n < K3 && live;
     const int c[3] = {n / K2, (n / K) % K, n % K};
-    if constexpr (LINES) {
-        // Line owners with their own face terms, storing their lines' results
-        // themselves (every value of G has one owner): one barrier per element.
-        constexpr int WPA = (K2 + 31) / 32;
-        const int w = n / 32, a = w / WPA, t = (w % WPA) * 32 + n % 32;
-        const bool owner = live && a < 3 && t < K2;
-        int code[2] = {0, 0};
-        if (owner) line_end_codes(m, e, a, code);
-        if constexpr (PDL) {
-            pdl_wait();
-            pdl_next();
-        }
-        T rho = T(0), ro[2] = {T(0), T(0)}, unused_u[2], unused_q[2];
-        if (act) rho = load_in<INCR, PDL>(io, 0, (size_t)e * io.np + n);
-        if (owner) line_end_values<INCR, false, false, PDL, T, K>(io, m, C, code, a, t, ro, unused_u, unused_q);
-        S.r[n] = rho;
-        __syncthreads();
-        if (owner) {
-            T* q = io.q_out + (size_t)a * io.fs + (size_t)e * io.np;
-            if (a == 0) grad_line_faces<0>(Cv, S, t, ro, q);
-            else if (a == 1) grad_line_faces<1>(Cv, S, t, ro, q);
-            else grad_line_faces<2>(Cv, S, t, ro, q);
-        }
-    } else {
-        // Face nodes assigned densely (see stage_kernel): their neighbour (or
-        // exterior) values are loaded with the thread's own node.
-        int code[R];
+    // Face nodes assigned densely (see stage_kernel): their neighbour (or
+    // exterior) values are loaded with the thread's own node.
+    int code[R];
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-            const int t = n + r * NPT;
-            code[r] = 0;
-            if (live && t < NF) {
-                const FaceNode<K> F(t);
-                code[r] = __ldg(m.nbr + (size_t)e * 6 + 2 * F.a + F.side);
-            }
-        }
-        if constexpr (PDL) {
-            pdl_wait();
-            pdl_next();
-        }
-        T rho = T(0);
-        if (act) rho = load_in<INCR, PDL>(io, 0, (size_t)e * io.np + n);
-        T ro[R];
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            ro[r] = T(0);
-            const int t = n + r * NPT;
-            if (!live || t >= NF) continue;
+    for (int r = 0; r < R; r++) {
+        const int t = n + r * NPT;
+        code[r] = 0;
+        if (live && t < NF) {
             const FaceNode<K> F(t);
-            if (code[r] >= 0) {
-                ro[r] = load_in<INCR, PDL>(io, 0, (size_t)code[r] * io.np + F.nn);
-            } else {
-                T uo;
-                exterior<T, K>(m, C, -1 - code[r], F.side, F.fi, ro[r], uo);
-            }
+            code[r] = __ldg(m.nbr + (size_t)e * 6 + 2 * F.a + F.side);
         }
-        OpRows<T, K> R_;
-        R_.load(C, c, act);
-        S.r[n] = rho;
-        __syncthreads();
+    }
+    T rho = T(0);
+    if (act) rho = load_in(io, 0, (size_t)e * io.np + n);
+    T ro[R];
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-            const int t = n + r * NPT;
-            if (!live || t >= NF) continue;
-            const FaceNode<K> F(t);
-            S.fl[F.a][F.side][F.fi] = ro[r] + S.r[F.nf];  // flux factors are in the lift columns
+    for (int r = 0; r < R; r++) {
+        ro[r] = T(0);
+        const int t = n + r * NPT;
+        if (!live || t >= NF) continue;
+        const FaceNode<K> F(t);
+        if (code[r] >= 0) {
+            ro[r] = load_in(io, 0, (size_t)code[r] * io.np + F.nn);
+        } else {
+            T uo;
+            exterior<T, K>(m, C, -1 - code[r], F.side, F.fi, ro[r], uo);
         }
-        __syncthreads();
-        if (!act) return;
+    }
+    OpRows<T, K> R_;
+    R_.load(C, c, act);
+    S.r[n] = rho;
+    __syncthreads();
 #pragma unroll
-        for (int a = 0; a < 3; a++) {
-            const int st = axis_stride<K>(a);
-            const int base = n - c[a] * st;
-            const int fi = c[(a + 1) % 3] * K + c[(a + 2) % 3];
-            T s = R_.l0[a] * S.fl[a][0][fi];
-            s += R_.ln[a] * S.fl[a][1][fi];
+    for (int r = 0; r < R; r++) {
+        const int t = n + r * NPT;
+        if (!live || t >= NF) continue;
+        const FaceNode<K> F(t);
+        S.fl[F.a][F.side][F.fi] = ro[r] + S.r[F.nf];  // flux factors are in the lift columns
+    }
+    __syncthreads();
+    if (!act) return;
 #pragma unroll
-            for (int j = 0; j < K; j++) s += R_.d[a][j] * S.r[base + j * st];
-            io.q_out[(size_t)a * io.fs + (size_t)e * io.np + n] = s;
-        }
+    for (int a = 0; a < 3; a++) {
+        const int st = axis_stride<K>(a);
+        const int base = n - c[a] * st;
+        const int fi = c[(a + 1) % 3] * K + c[(a + 2) % 3];
+        T s = R_.l0[a] * S.fl[a][0][fi];
+        s += R_.ln[a] * S.fl[a][1][fi];
+#pragma unroll
+        for (int j = 0; j < K; j++) s += R_.d[a][j] * S.r[base + j * st];
+        io.q_out[(size_t)a * io.fs + (size_t)e * io.np + n] = s;
     }
 }
 
@@ -570,7 +408,7 @@ ldg_gradient_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict
 // (f_mom, f_mass along a + G_a) of every node (one 8- or 16-byte load feeds
 // two FMAs of a line sum), the pair (momentum, density) of every face term
 // [axis][side][face node], and each node's own mass flux and gradient, which
-// the face phase reads (and the FP32 line owners then reuse for their results).
+// the face phase reads (and the batch's line owners reuse for their results).
 template <typename T, int K>
 struct PlainSmem {
     typename Pair<T>::type f[3][npt_of(K)];
@@ -650,9 +488,9 @@ stage_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__ Cp, 
     T fl[4] = {T(0), T(0), T(0), T(0)};
     if (act) {
         if (FLUX != 2) {  // mode 2 needs the state only for the stage combination
-            rho = load_in<false>(io, 0, off);
+            rho = load_in(io, 0, off);
 #pragma unroll
-            for (int a = 0; a < 3; a++) u[a] = load_in<false>(io, 1 + a, off);
+            for (int a = 0; a < 3; a++) u[a] = load_in(io, 1 + a, off);
         }
         if (DIFF)
 #pragma unroll
@@ -678,8 +516,8 @@ stage_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__ Cp, 
                 ro[r] = __ldg(io.flux_in + o2);
                 uo[r] = __ldg(io.flux_in + (size_t)(1 + F.a) * io.fs + o2);
             } else {
-                ro[r] = load_in<false>(io, 0, o2);
-                uo[r] = load_in<false>(io, 1 + F.a, o2);
+                ro[r] = load_in(io, 0, o2);
+                uo[r] = load_in(io, 1 + F.a, o2);
             }
             if (DIFF) qo[r] = __ldg(io.q + (size_t)F.a * io.fs + o2);
         } else {
@@ -747,9 +585,9 @@ stage_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__ Cp, 
     // no thread spends FP64 instructions on it; computed here when absent.
     const T cbe = io.elem_b ? __ldg(io.elem_b + e) : io.cb - (do_sponge ? io.ca * __ldg(m.sigma + e) : T(0));
     if (FLUX == 2) {
-        rho = load_in<false>(io, 0, off);
+        rho = load_in(io, 0, off);
 #pragma unroll
-        for (int a = 0; a < 3; a++) u[a] = load_in<false>(io, 1 + a, off);
+        for (int a = 0; a < 3; a++) u[a] = load_in(io, 1 + a, off);
     }
 
     const T r[4] = {r_rho, r_u[0], r_u[1], r_u[2]};
@@ -769,202 +607,6 @@ stage_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__ Cp, 
 #pragma unroll
         for (int a = 0; a < 3; a++)
             io.flux_out[(size_t)(1 + a) * io.fs + off] = mass_flux(vo[1 + a], vo[0], C.r0, C.linear_mass);
-    }
-}
-
-// ---------------------------------------------------------------------------
-// One RK stage of the increment (FP32) form.  The kernel waits on memory
-// latency and on the L1 data pipe, so every global load a thread makes is
-// issued before the first value is used (face-table codes and sigma, its own
-// u, d, gradient and Kahan compensation, the neighbour values of its face
-// nodes), and the face nodes are assigned densely as in stage_kernel, which
-// also makes the neighbour gathers denser warp requests.  The face fluxes are
-// evaluated after a barrier from the element's own values in shared memory.
-//
-// The line sums (the L1 data pipe's largest load: 2 (K + 2) shared-memory
-// operands per node and axis when each node sums its own lines) are done by
-// line owners for K >= 5: warps take one axis each, a lane one line of the
-// element, reads the line's K flux pairs and two face terms once and produces
-// all K outputs, with the operator rows taken from kernel-parameter space
-// (``Cv``; warp-uniform indices, so constant-bank operands).  The per-axis
-// results go to shared memory and each node thread adds them up.
-// ---------------------------------------------------------------------------
-// Resident CTAs per SM asked of the compiler for the FP32 stage kernel (0: no
-// request): at K = 5 it fits 40 registers without spilling, 12 CTAs per SM.
-template <typename T, int K>
-__host__ __device__ constexpr int incr_min_blocks()
-{
-    return (sizeof(T) == 4 && K == 5) ? 12 : 0;
-}
-
-template <typename T, int K, bool DIFF, bool PDL>
-__global__ void __launch_bounds__(npt_of(K) * epb_of(K), (incr_min_blocks<T, K>()))
-incr_stage_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__ Cp, const OpConst<T, K> Cv,
-                  int do_adv, int do_sponge)
-{
-    constexpr bool LINES = K >= 5;  // three warp-groups of ceil(K^2 / 32) warps fit in NPT
-    constexpr int K2 = K * K, K3 = K * K * K, NPT = npt_of(K), NF = 6 * K2, R = (NF + NPT - 1) / NPT;
-    constexpr int WPA = (K2 + 31) / 32;
-    __shared__ PlainSmem<T, K> sm_all[epb_of(K)];
-    PlainSmem<T, K>& S = sm_all[threadIdx.y];
-    const OpConst<T, K>& C = *Cp;
-    const int n = threadIdx.x;
-    const int e = blockIdx.x * epb_of(K) + threadIdx.y;
-    const bool live = e < m.n_elem;
-    const bool act = n < K3 && live;
-    const int c[3] = {n / K2, (n / K) % K, n % K};
-    const size_t off = (size_t)e * io.np + n;
-    // line owner (LINES): warp group a, line t of that axis
-    const int la = n / 32 / WPA, lt = (n / 32 % WPA) * 32 + n % 32;
-    const bool owner = LINES && live && la < 3 && lt < K2;
-
-    int code[R > 2 ? R : 2] = {0, 0};
-    if constexpr (LINES) {
-        if (owner) line_end_codes(m, e, la, code);
-    } else {
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            const int t = n + r * NPT;
-            code[r] = 0;
-            if (live && t < NF) {
-                const FaceNode<K> F(t);
-                code[r] = __ldg(m.nbr + (size_t)e * 6 + 2 * F.a + F.side);
-            }
-        }
-    }
-    const T sig = (act && do_sponge) ? __ldg(m.sigma + e) : T(0);
-    if constexpr (PDL) {
-        pdl_wait();
-        pdl_next();
-    }
-    T ub[4] = {T(0), T(0), T(0), T(0)}, dv[4] = {T(0), T(0), T(0), T(0)};
-    T cmp[4] = {T(0), T(0), T(0), T(0)}, q[3] = {T(0), T(0), T(0)};
-    if (act) {
-#pragma unroll
-        for (int f = 0; f < 4; f++) {
-            ub[f] = pdl_load<PDL>(io.src + (size_t)f * io.fs + off);
-            if (io.inc) dv[f] = pdl_load<PDL>(io.inc + (size_t)f * io.fs + off);
-            if (io.final_stage) cmp[f] = io.comp[(size_t)f * io.fs + off];
-        }
-        if (DIFF)
-#pragma unroll
-            for (int a = 0; a < 3; a++) q[a] = pdl_load<PDL>(io.q + (size_t)a * io.fs + off);
-    }
-    // Neighbour (or exterior) values: of the two ends of the owned line
-    // (LINES), else of the densely assigned face nodes.
-    T ro[R > 2 ? R : 2], uo[R > 2 ? R : 2], qo[R > 2 ? R : 2];
-    if constexpr (LINES) {
-        if (owner) line_end_values<true, true, DIFF, PDL, T, K>(io, m, C, code, la, lt, ro, uo, qo);
-    } else {
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            ro[r] = uo[r] = qo[r] = T(0);
-            const int t = n + r * NPT;
-            if (!live || t >= NF) continue;
-            const FaceNode<K> F(t);
-            if (code[r] >= 0) {
-                const size_t o2 = (size_t)code[r] * io.np + F.nn;
-                ro[r] = load_in<true, PDL>(io, 0, o2);
-                uo[r] = load_in<true, PDL>(io, 1 + F.a, o2);
-                if (DIFF) qo[r] = pdl_load<PDL>(io.q + (size_t)F.a * io.fs + o2);
-            } else {
-                exterior<T, K>(m, C, -1 - code[r], F.side, F.fi, ro[r], uo[r]);
-            }
-        }
-    }
-    OpRows<T, K> R_;
-    if constexpr (!LINES) R_.load(C, c, act);
-
-    const T rho = ub[0] + dv[0];
-    const T u[3] = {ub[1] + dv[1], ub[2] + dv[2], ub[3] + dv[3]};
-    T fmom = T(0), fmass[3] = {T(0), T(0), T(0)};
-    if (do_adv) {
-        fmom = momentum_flux(rho, C.k1, C.k2);
-#pragma unroll
-        for (int a = 0; a < 3; a++) fmass[a] = mass_flux(u[a], rho, C.r0, C.linear_mass);
-    }
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        S.f[a][n].x = fmom;
-        S.f[a][n].y = DIFF ? fmass[a] + q[a] : fmass[a];
-        S.m[a][n] = fmass[a];
-        if (DIFF) S.q[a][n] = q[a];
-    }
-    __syncthreads();
-
-    T r[4] = {T(0), T(0), T(0), T(0)};
-    if constexpr (LINES) {
-        // Line owners evaluate the face terms at both ends of their line and
-        // the line sums; the per-axis results reuse S.m (density) and S.q
-        // (momentum) of the owner's own line nodes, read before written.
-        if (owner) {
-            if (la == 0) stage_line_faces<0, DIFF>(Cv, S, lt, ro, uo, qo, do_adv);
-            else if (la == 1) stage_line_faces<1, DIFF>(Cv, S, lt, ro, uo, qo, do_adv);
-            else stage_line_faces<2, DIFF>(Cv, S, lt, ro, uo, qo, do_adv);
-        }
-        __syncthreads();
-        if (!act) return;
-#pragma unroll
-        for (int a2 = 0; a2 < 3; a2++) {
-            r[0] += S.m[a2][n];
-            r[1 + a2] = do_adv ? S.q[a2][n] : T(0);
-        }
-    } else {
-#pragma unroll
-        for (int rr = 0; rr < R; rr++) {
-            const int t = n + rr * NPT;
-            if (!live || t >= NF) continue;
-            const FaceNode<K> F(t);
-            const T fm_s = S.f[F.a][F.nf].x, fa_s = S.m[F.a][F.nf];
-            T gm = T(0), gr = T(0);
-            if (do_adv) {
-                const T fmo = momentum_flux(ro[rr], C.k1, C.k2);
-                const T fao = mass_flux(uo[rr], ro[rr], C.r0, C.linear_mass);
-                const T* cm = C.cM[F.a][F.side];
-                const T* cr = C.cA[F.a][F.side];
-                gm = fmo * cm[0] + fm_s * cm[1] + fao * cm[2] + fa_s * cm[3];
-                gr = fmo * cr[0] + fm_s * cr[1] + fao * cr[2] + fa_s * cr[3];
-            }
-            if (DIFF) gr += C.cQ[F.a][F.side] * (qo[rr] + S.q[F.a][F.nf]);
-            S.g[F.a][F.side][F.fi].x = gm;
-            S.g[F.a][F.side][F.fi].y = gr;
-        }
-        __syncthreads();
-        if (!act) return;
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            const int st = axis_stride<K>(a), base = n - c[a] * st;
-            const int fi = c[(a + 1) % 3] * K + c[(a + 2) % 3];
-            const typename Pair<T>::type g0 = S.g[a][0][fi], gN = S.g[a][1][fi];
-            T sm = R_.l0[a] * g0.x, sr = R_.l0[a] * g0.y;
-            sm += R_.ln[a] * gN.x;
-            sr += R_.ln[a] * gN.y;
-#pragma unroll
-            for (int j = 0; j < K; j++) {
-                const typename Pair<T>::type v = S.f[a][base + j * st];
-                sm += R_.d[a][j] * v.x;
-                sr += R_.d[a][j] * v.y;
-            }
-            r[0] += sr;
-            r[1 + a] = do_adv ? sm : T(0);
-        }
-    }
-    const T ks = io.ca * sig;
-    const T cbe = io.cb - ks, ce = io.eps - ks;
-#pragma unroll
-    for (int f = 0; f < 4; f++) {
-        const size_t o = (size_t)f * io.fs + off;
-        T d = r[f] + ub[f] * ce;
-        if (io.inc) d += dv[f] * cbe;
-        if (io.final_stage) {
-            // Kahan-compensated u <- u + d
-            const T y = d - cmp[f];
-            const T t = ub[f] + y;
-            io.comp[o] = (t - ub[f]) - y;
-            io.dst[o] = t;
-        } else {
-            io.dst[o] = d;
-        }
     }
 }
 

@@ -14,6 +14,7 @@
 #include "dg3d.h"
 #include "dg_kernels.cuh"
 #include "fix_kernels.cuh"
+#include "incr_kernels.cuh"
 #include "mesh.h"
 #include "solver_internal.h"
 
@@ -62,13 +63,13 @@ double grad_flops(const Solver& s)
     return (3.0 * 2.0 * (K + 2.0) + 6.0 / K * 2.0) * (double)s.gsize();
 }
 
-template <typename T, bool INCR>
+template <typename T>
 double stage_bytes(const Solver& s, const StageIO<T>& io)
 {
     const double nn = (double)s.gsize();
     const double diff = s.p.eval_diff ? 3.0 : 0.0;
     double vals;
-    if (!INCR) vals = 4.0 + diff + (io.old ? 4.0 : 0.0) + 4.0;
+    if (sizeof(T) == 8) vals = 4.0 + diff + (io.old ? 4.0 : 0.0) + 4.0;
     else vals = 4.0 + (io.inc ? 4.0 : 0.0) + diff + 4.0 + (io.final_stage ? 8.0 : 0.0);
     return vals * sizeof(T) * nn;
 }
@@ -151,28 +152,24 @@ const OpConst<T, K>* const_ptr(const Solver& s, int slot)
     return (const OpConst<T, K>*)((const char*)s.d_const + (size_t)slot * const_slot<T, K>());
 }
 
-template <typename T, int K, bool INCR>
+template <typename T, int K>
 void launch_grad(Solver& s, const StageIO<T>& io, const MeshDev<T>& md)
 {
-    dim3 block(npt_of(K), epb_of(K));
-    dim3 grid((md.n_elem + epb_of(K) - 1) / epb_of(K));
     cudaEvent_t ev = nullptr;
     s.prof_begin(1, &ev);
-    bool done = false;
-    if constexpr (!INCR && sizeof(T) == 8) {
-        if (s.fix_ok[3]) {
-            launch_pdl(ldg_gradient_fix_kernel<K>, (md.n_elem + fix_epb(K) - 1) / fix_epb(K), fix_threads(K), s.stream,
-                       io, md, host_const<T, K>(s, 3), fix_set<K>(s).grad);
-            done = true;
-        }
-    }
-    if (!done)
+    if constexpr (sizeof(T) == 4) {
+        const int grid = (md.n_elem + incr_epb(K) - 1) / incr_epb(K);
         if (s.short_launches())
-            launch_pdl(ldg_gradient_kernel<T, K, INCR, true>, grid, block, s.stream, io, md, const_ptr<T, K>(s, 3),
-                       host_const<T, K>(s, 3));
+            launch_pdl(incr_gradient_kernel<K, true>, grid, incr_threads(K), s.stream, io, md, host_const<T, K>(s, 3));
         else
-            ldg_gradient_kernel<T, K, INCR, false><<<grid, block, 0, s.stream>>>(io, md, const_ptr<T, K>(s, 3),
-                                                                                host_const<T, K>(s, 3));
+            incr_gradient_kernel<K, false><<<grid, incr_threads(K), 0, s.stream>>>(io, md, host_const<T, K>(s, 3));
+    } else if (s.fix_ok[3]) {
+        launch_pdl(ldg_gradient_fix_kernel<K>, (md.n_elem + fix_epb(K) - 1) / fix_epb(K), fix_threads(K), s.stream, io,
+                   md, host_const<T, K>(s, 3), fix_set<K>(s).grad);
+    } else {
+        ldg_gradient_kernel<T, K><<<(md.n_elem + epb_of(K) - 1) / epb_of(K), dim3(npt_of(K), epb_of(K)), 0, s.stream>>>(
+            io, md, const_ptr<T, K>(s, 3));
+    }
     s.prof_end(1, ev, grad_bytes(s, io), grad_flops(s));
     s.launches++;
 }
@@ -209,35 +206,38 @@ void launch_plain(const Solver& s, int slot, const StageIO<double>& io, const Me
     }
 }
 
-template <typename T, int K, bool DIFF>
-void launch_incr(const Solver& s, dim3 grid, dim3 block, const StageIO<T>& io, const MeshDev<T>& md,
-                 const OpConst<T, K>* Cp, const OpConst<T, K>& Cv)
+template <int K, bool DIFF, bool PDL>
+constexpr auto incr_stage()
 {
-    if (s.short_launches())
-        launch_pdl(incr_stage_kernel<T, K, DIFF, true>, grid, block, s.stream, io, md, Cp, Cv, s.p.eval_advect,
-                   s.p.eval_sponge);
-    else
-        incr_stage_kernel<T, K, DIFF, false><<<grid, block, 0, s.stream>>>(io, md, Cp, Cv, s.p.eval_advect,
-                                                                           s.p.eval_sponge);
+    if constexpr (incr_epb(K) > 1) return incr_packed_stage_kernel<K, DIFF, PDL>;
+    else return incr_stage_kernel<K, DIFF, PDL>;
 }
 
-template <typename T, int K, bool INCR>
+template <int K, bool DIFF>
+void launch_incr(const Solver& s, const StageIO<float>& io, const MeshDev<float>& md, const OpConst<float, K>& C)
+{
+    const int grid = (md.n_elem + incr_epb(K) - 1) / incr_epb(K);
+    if (s.short_launches())
+        launch_pdl(incr_stage<K, DIFF, true>(), grid, incr_threads(K), s.stream, io, md, C, s.p.eval_advect,
+                   s.p.eval_sponge);
+    else
+        incr_stage<K, DIFF, false>()<<<grid, incr_threads(K), 0, s.stream>>>(io, md, C, s.p.eval_advect,
+                                                                              s.p.eval_sponge);
+}
+
+template <typename T, int K>
 void launch_stage(Solver& s, const StageIO<T>& io, const MeshDev<T>& md, int slot)
 {
     cudaEvent_t ev = nullptr;
     s.prof_begin(0, &ev);
-    if constexpr (INCR) {
-        const OpConst<T, K>* Cp = const_ptr<T, K>(s, slot);
-        const dim3 block(npt_of(K), epb_of(K));
-        const dim3 grid((md.n_elem + epb_of(K) - 1) / epb_of(K));
-        const OpConst<T, K>& Cv = host_const<T, K>(s, slot);
-        if (s.p.eval_diff) launch_incr<T, K, true>(s, grid, block, io, md, Cp, Cv);
-        else launch_incr<T, K, false>(s, grid, block, io, md, Cp, Cv);
+    if constexpr (sizeof(T) == 4) {
+        if (s.p.eval_diff) launch_incr<K, true>(s, io, md, host_const<T, K>(s, slot));
+        else launch_incr<K, false>(s, io, md, host_const<T, K>(s, slot));
     } else {
         if (s.p.eval_diff) launch_plain<K, true>(s, slot, io, md);
         else launch_plain<K, false>(s, slot, io, md);
     }
-    s.prof_end(0, ev, stage_bytes<T, INCR>(s, io), stage_flops(s, io.old != nullptr || io.inc != nullptr));
+    s.prof_end(0, ev, stage_bytes(s, io), stage_flops(s, io.old != nullptr || io.inc != nullptr));
     s.launches++;
 }
 
@@ -281,31 +281,31 @@ int upload_consts(Solver& s, double dt)
     return fail(DG_ERR_INVALID, "unsupported order");
 }
 
-template <typename T, bool INCR>
+template <typename T>
 void dispatch_grad(Solver& s, const StageIO<T>& io, const MeshDev<T>& md)
 {
     switch (s.mesh.K) {
-    case 2: launch_grad<T, 2, INCR>(s, io, md); break;
-    case 3: launch_grad<T, 3, INCR>(s, io, md); break;
-    case 4: launch_grad<T, 4, INCR>(s, io, md); break;
-    case 5: launch_grad<T, 5, INCR>(s, io, md); break;
-    case 6: launch_grad<T, 6, INCR>(s, io, md); break;
-    case 7: launch_grad<T, 7, INCR>(s, io, md); break;
-    case 8: launch_grad<T, 8, INCR>(s, io, md); break;
+    case 2: launch_grad<T, 2>(s, io, md); break;
+    case 3: launch_grad<T, 3>(s, io, md); break;
+    case 4: launch_grad<T, 4>(s, io, md); break;
+    case 5: launch_grad<T, 5>(s, io, md); break;
+    case 6: launch_grad<T, 6>(s, io, md); break;
+    case 7: launch_grad<T, 7>(s, io, md); break;
+    case 8: launch_grad<T, 8>(s, io, md); break;
     }
 }
 
-template <typename T, bool INCR>
+template <typename T>
 void dispatch_stage(Solver& s, const StageIO<T>& io, const MeshDev<T>& md, int slot)
 {
     switch (s.mesh.K) {
-    case 2: launch_stage<T, 2, INCR>(s, io, md, slot); break;
-    case 3: launch_stage<T, 3, INCR>(s, io, md, slot); break;
-    case 4: launch_stage<T, 4, INCR>(s, io, md, slot); break;
-    case 5: launch_stage<T, 5, INCR>(s, io, md, slot); break;
-    case 6: launch_stage<T, 6, INCR>(s, io, md, slot); break;
-    case 7: launch_stage<T, 7, INCR>(s, io, md, slot); break;
-    case 8: launch_stage<T, 8, INCR>(s, io, md, slot); break;
+    case 2: launch_stage<T, 2>(s, io, md, slot); break;
+    case 3: launch_stage<T, 3>(s, io, md, slot); break;
+    case 4: launch_stage<T, 4>(s, io, md, slot); break;
+    case 5: launch_stage<T, 5>(s, io, md, slot); break;
+    case 6: launch_stage<T, 6>(s, io, md, slot); break;
+    case 7: launch_stage<T, 7>(s, io, md, slot); break;
+    case 8: launch_stage<T, 8>(s, io, md, slot); break;
     }
 }
 
@@ -397,8 +397,8 @@ int Solver::rk_stage_fp64(int s_idx, double dt, double* rhs_only)
         io.pack_gsize = gsize();
         stage3_packed = true;
     }
-    if (p.eval_diff) dispatch_grad<double, false>(*this, io, md);
-    dispatch_stage<double, false>(*this, io, md, rhs_only ? 4 : s_idx);
+    if (p.eval_diff) dispatch_grad<double>(*this, io, md);
+    dispatch_stage<double>(*this, io, md, rhs_only ? 4 : s_idx);
     if (fluxes) {
         flux_cur = 1 - flux_cur;
         flux_valid = true;
@@ -447,8 +447,8 @@ int Solver::rk_stage_fp32(int s_idx, double dt, float* rhs_only)
         if (rc) return rc;
     }
     (void)ca;
-    if (p.eval_diff) dispatch_grad<float, true>(*this, io, md);
-    dispatch_stage<float, true>(*this, io, md, rhs_only ? 4 : s_idx);
+    if (p.eval_diff) dispatch_grad<float>(*this, io, md);
+    dispatch_stage<float>(*this, io, md, rhs_only ? 4 : s_idx);
     return DG_OK;
 }
 
