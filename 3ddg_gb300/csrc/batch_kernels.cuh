@@ -107,6 +107,14 @@ __device__ __forceinline__ bool batch_line_task(int slot, int n, int& ls, int& a
     return ls < EPB && a < 3 && t < K2;
 }
 
+// First node of line t along axis a, t = the two other coordinates with z
+// varying fastest where it is one of them.
+template <int K>
+__device__ __forceinline__ int batch_line_node(int a, int t)
+{
+    return a == 0 ? t : (a == 1 ? t / K * K * K + t % K : t * K);
+}
+
 // Face-table codes of the two ends of the owner's line (element c0 + ls).
 template <int K>
 __device__ __forceinline__ void batch_end_codes(const BatchProblem& P, const BatchTile& T, int c0, bool task, int ls,
@@ -134,9 +142,9 @@ struct BatchGradSmem {
 // are loaded during the pass before.
 template <int K, bool PDL>
 __device__ void batch_grad_tile(const BatchProblem& P, const BatchOps& ops, const BatchTile& T, int stage,
-                                unsigned char* smraw)
+                                bool wait, unsigned char* smraw)
 {
-    constexpr int K2 = K * K, K3 = K * K * K, NPT = npt_of(K), EPB = bepb_of(K);
+    constexpr int K3 = K * K * K, NPT = npt_of(K), EPB = bepb_of(K);
     BatchGradSmem<K>* SM = reinterpret_cast<BatchGradSmem<K>*>(smraw);
     const int slot = threadIdx.x / NPT, n = threadIdx.x % NPT;
     const float* ub = P.u[P.cur];
@@ -144,9 +152,13 @@ __device__ void batch_grad_tile(const BatchProblem& P, const BatchOps& ops, cons
     int ls = 0, a = 0, t = 0;
     const bool task = batch_line_task<K>(slot, n, ls, a, t);
     const int st = axis_stride<K>(a < 3 ? a : 0);
-    const int b0 = a == 0 ? t : (a == 1 ? (t % K) * K2 + (t / K) : t * K);
+    const int b0 = batch_line_node<K>(a, t);
     int code_next[2];
     batch_end_codes<K>(P, T, T.e0, task, ls, a, code_next);
+    if (PDL && wait) {
+        pdl_wait();
+        pdl_next();
+    }
     int buf = 0;
     for (int c0 = T.e0; c0 < T.e0 + T.count; c0 += EPB, buf ^= 1) {
         const int e = c0 + slot;
@@ -195,7 +207,7 @@ __device__ void batch_grad_tile(const BatchProblem& P, const BatchOps& ops, cons
 
 template <int K, bool PDL>
 __device__ void batch_stage_tile(const BatchProblem& P, const BatchOps& ops, const BatchTile& T, int stage,
-                                 unsigned char* smraw)
+                                 bool wait, unsigned char* smraw)
 {
     constexpr int K2 = K * K, K3 = K * K * K, NPT = npt_of(K), EPB = bepb_of(K), NF = 6 * K2;
     constexpr int R = (NF + NPT - 1) / NPT;
@@ -212,6 +224,10 @@ __device__ void batch_stage_tile(const BatchProblem& P, const BatchOps& ops, con
     int code_next[R];
     batch_codes<K, R>(P, T, T.e0, slot, n, code_next);
     float sig_next = batch_sigma<K>(P, T, T.e0, slot, n);
+    if (PDL && wait) {
+        pdl_wait();
+        pdl_next();
+    }
     for (int c0 = T.e0; c0 < T.e0 + T.count; c0 += EPB) {
         const int e = c0 + slot;
         const bool live = slot < EPB && e < T.e0 + T.count;
@@ -314,11 +330,11 @@ __device__ void batch_stage_tile(const BatchProblem& P, const BatchOps& ops, con
             PlainSmem<float, K>& S = SM[ls < EPB ? ls : 0];
             if (ls < EPB && c0 + ls < T.e0 + T.count && a < 3 && t < K2) {
                 const int st = axis_stride<K>(a);
-                const int b0 = a == 0 ? t : (a == 1 ? (t % K) * K2 + (t / K) : t * K);
+                const int b0 = batch_line_node<K>(a, t), fi = a == 1 ? t % K * K + t / K : t;
                 float2 v[K];
 #pragma unroll
                 for (int j = 0; j < K; j++) v[j] = S.f[a][b0 + j * st];
-                const float2 g0 = S.g[a][0][t], gN = S.g[a][1][t];
+                const float2 g0 = S.g[a][0][fi], gN = S.g[a][1][fi];
                 const float iw = P.invw[a];
 #pragma unroll
                 for (int i = 0; i < K; i++) {
@@ -420,16 +436,13 @@ __global__ void __launch_bounds__(bthreads_of(K), batch_min_blocks(K, PHASE))
     for (int ti = blockIdx.x; ti < A.n_tiles;) {
         const BatchTile T = A.tiles[A.tile0 + ti];
         load_problem(P, A.probs + T.prob);
-        if (first) {
-            // tiles, counters and descriptors are the same for all kernels of a step
-            pdl_wait();
-            pdl_next();
-            first = false;
-        }
         __syncthreads();
+        // tiles, counters, descriptors and face tables are the same for all
+        // kernels of a step: the wait for the kernel before comes after them
         if (P.active) {
-            if constexpr (PHASE == 0) batch_grad_tile<K, PDL>(P, ops, T, A.stage, smraw);
-            else batch_stage_tile<K, PDL>(P, ops, T, A.stage, smraw);
+            if constexpr (PHASE == 0) batch_grad_tile<K, PDL>(P, ops, T, A.stage, first, smraw);
+            else batch_stage_tile<K, PDL>(P, ops, T, A.stage, first, smraw);
+            first = false;
         }
         if (A.n_tiles <= gridDim.x) break;
         if (threadIdx.x == 0) tile_idx = gridDim.x + atomicAdd(A.counters + PHASE, 1);

@@ -16,7 +16,7 @@
 
 namespace dg {
 
-__host__ __device__ constexpr int fix_epb(int K) { return K == 2 ? 16 : K == 3 ? 9 : K == 4 ? 4 : K == 5 ? 2 : 1; }
+__host__ __device__ constexpr int fix_epb(int K) { return K == 2 ? 16 : K == 3 ? 9 : K <= 5 ? 2 : 1; }
 __host__ __device__ constexpr int fix_threads(int K) { return (fix_epb(K) * K * K * K + 31) / 32 * 32; }
 __host__ __device__ constexpr int fix_rounds(int K)
 {
@@ -342,17 +342,20 @@ __device__ __forceinline__ void stage_fix_line(const OpConst<double, K>& C, cons
 }
 
 // What bounds these kernels and what they measured (ms per launch at 32.8 M
-// nodes, sums of even-odd or per-node FP64 lines -> fixed point):
+// nodes, even-odd or per-node FP64 line sums -> fixed point):
 //   K          2           3           4           5           6           7           8
-//   stage      8.99->1.52  4.49->1.50  3.85->1.32  3.85->1.39  4.28->1.53  4.69->1.76  5.67->1.65
-//   gradient   1.54->0.56  1.10->0.44  1.11->0.48  1.11->0.48  1.40->0.56  1.60->0.56  1.69->0.57
+//   stage      8.99->1.44  4.49->1.43  3.85->1.21  3.85->1.35  4.28->1.47  4.69->1.67  5.67->1.56
+//   gradient   1.54->0.57  1.10->0.42  1.11->0.43  1.11->0.41  1.40->0.52  1.60->0.53  1.69->0.54
 // At K = 5 a stage launch keeps the FP64 pipe about 62 % busy (16 operations per
 // node), the integer pipe 50 %, the issue slots 60 % and HBM at 65 % of a copy:
 // no unit is the bound by itself, the barriers between the node and line phases
 // are (26 % of the warps' time), so resident warps count most.  Registers per
-// thread of the stage kernel, chosen by that (K = 5: 367 us per launch on 8 M
-// nodes at 48, 383 at 40, 392 at 56, 537 at 80 with an earlier form).
-__host__ __device__ constexpr int fix_regs(int K) { return K == 3 || K == 8 ? 40 : K == 6 ? 56 : 48; }
+// thread of the stage kernel and elements per CTA were chosen by that (us per
+// launch on 8 M nodes: K = 5 at 40 / 48 / 56 / 80 registers 335 / 329 / 358 /
+// 537; K = 8 at 32 / 40 / 48 380 / 404 / 494; K = 4 at 1 / 2 / 4 / 6 elements
+// 383 / 296 / 311 / 349).  Converting results on the FP64 pipe (fix_to_fp64)
+// instead saves integer work where that pipe is the scarcer one: 346 for 329 us.
+__host__ __device__ constexpr int fix_regs(int K) { return K == 8 ? 32 : K == 6 ? 56 : 48; }
 __host__ __device__ constexpr int fix_min_blocks(int K) { return 65536 / (fix_regs(K) * fix_threads(K)); }
 // The stage input and the old state are fetched into shared memory at the
 // start where they fit beside the line data.
