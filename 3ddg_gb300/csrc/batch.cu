@@ -71,19 +71,23 @@ void fill_ops(BatchProblem& P, const LineOperators& op, const dg_params& p)
     P.linear_mass = C.linear_mass;
 }
 
-// A launch whose blocks take few tiles each starts under the one before it in
-// its branch (launch_pdl; with the step bookkeeping in one launch, 8 problems of 4..8 elements per axis 53 -> 43 us per
-// step, one of 6^3 32 -> 20 us); one that streams many has no gap to hide and
-// keeps the read-only loads.  The first launch of a step (``after`` false)
-// reads descriptors that the launch before it wrote, so it waits for it.
-constexpr int kDependentTiles = 2;
+// A launch with a block for every tile starts under the one before it in its
+// branch (launch_pdl; with the step bookkeeping in one launch, 8 problems of
+// 4..8 elements per axis 53 -> 42 us per step, one of 6^3 32 -> 20 us); one
+// whose blocks stream several has no gap to hide and keeps the read-only loads
+// and the smaller register budget (24 uneven problems, about two tiles per
+// block: 581 us per step when launched so, 529 when not).  The first launch of
+// a step (``after`` false) reads descriptors that the launch before it wrote,
+// so it waits for it.
 template <int K, int PHASE>
-void launch_batch(const BatchArgs& A, const BatchOps& ops, int grid, bool after, cudaStream_t st)
+void launch_batch(const BatchArgs& A, const BatchOps& ops, int grid, bool after, bool narrow, cudaStream_t st)
 {
-    if (after && A.n_tiles <= kDependentTiles * grid)
-        launch_pdl(batch_stage_kernel<K, PHASE, true>, grid, bthreads_of(K), st, A, ops);
+    if (!narrow)
+        batch_stage_kernel<K, PHASE, false, size_t><<<grid, bthreads_of(K), 0, st>>>(A, ops);
+    else if (after && A.n_tiles <= grid)
+        launch_pdl(batch_stage_kernel<K, PHASE, true, unsigned>, grid, bthreads_of(K), st, A, ops);
     else
-        batch_stage_kernel<K, PHASE, false><<<grid, bthreads_of(K), 0, st>>>(A, ops);
+        batch_stage_kernel<K, PHASE, false, unsigned><<<grid, bthreads_of(K), 0, st>>>(A, ops);
 }
 
 }  // namespace
@@ -188,16 +192,16 @@ int Batch::init(int device_capacity)
     cudaDeviceProp prop;
     DGB_CUDA(cudaGetDeviceProperties(&prop, device));
     num_sms = prop.multiProcessorCount;
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[2][0], batch_stage_kernel<2, 0, false>, bthreads_of(2), 0));
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[2][1], batch_stage_kernel<2, 1, false>, bthreads_of(2), 0));
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[3][0], batch_stage_kernel<3, 0, false>, bthreads_of(3), 0));
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[3][1], batch_stage_kernel<3, 1, false>, bthreads_of(3), 0));
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[4][0], batch_stage_kernel<4, 0, false>, bthreads_of(4), 0));
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[4][1], batch_stage_kernel<4, 1, false>, bthreads_of(4), 0));
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[5][0], batch_stage_kernel<5, 0, false>, bthreads_of(5), 0));
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[5][1], batch_stage_kernel<5, 1, false>, bthreads_of(5), 0));
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[6][0], batch_stage_kernel<6, 0, false>, bthreads_of(6), 0));
-    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[6][1], batch_stage_kernel<6, 1, false>, bthreads_of(6), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[2][0], batch_stage_kernel<2, 0, false, unsigned>, bthreads_of(2), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[2][1], batch_stage_kernel<2, 1, false, unsigned>, bthreads_of(2), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[3][0], batch_stage_kernel<3, 0, false, unsigned>, bthreads_of(3), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[3][1], batch_stage_kernel<3, 1, false, unsigned>, bthreads_of(3), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[4][0], batch_stage_kernel<4, 0, false, unsigned>, bthreads_of(4), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[4][1], batch_stage_kernel<4, 1, false, unsigned>, bthreads_of(4), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[5][0], batch_stage_kernel<5, 0, false, unsigned>, bthreads_of(5), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[5][1], batch_stage_kernel<5, 1, false, unsigned>, bthreads_of(5), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[6][0], batch_stage_kernel<6, 0, false, unsigned>, bthreads_of(6), 0));
+    DGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_k[6][1], batch_stage_kernel<6, 1, false, unsigned>, bthreads_of(6), 0));
     max_ctas_per_sm = 1;
     for (int k = 2; k <= BATCH_KMAX; k++) {
         for (int ph = 0; ph < 2; ph++) {
@@ -494,6 +498,7 @@ void Batch::build_tiles()
             tiles.push_back(t);
         }
         groups.back().end = (int)tiles.size();
+        groups.back().narrow = groups.back().narrow && batch_narrow(E.fs);
     }
 }
 
@@ -566,16 +571,16 @@ int Batch::launch_step()
                     std::max(1, std::min(num_sms * std::min(ctas_per_sm, occ_k[K][phase]), A.n_tiles));
                 const bool after = s + phase > 0;
                 switch (K * 2 + phase) {
-                case 4: launch_batch<2, 0>(A, grp.ops, grid, after, bs); break;
-                case 5: launch_batch<2, 1>(A, grp.ops, grid, after, bs); break;
-                case 6: launch_batch<3, 0>(A, grp.ops, grid, after, bs); break;
-                case 7: launch_batch<3, 1>(A, grp.ops, grid, after, bs); break;
-                case 8: launch_batch<4, 0>(A, grp.ops, grid, after, bs); break;
-                case 9: launch_batch<4, 1>(A, grp.ops, grid, after, bs); break;
-                case 10: launch_batch<5, 0>(A, grp.ops, grid, after, bs); break;
-                case 11: launch_batch<5, 1>(A, grp.ops, grid, after, bs); break;
-                case 12: launch_batch<6, 0>(A, grp.ops, grid, after, bs); break;
-                case 13: launch_batch<6, 1>(A, grp.ops, grid, after, bs); break;
+                case 4: launch_batch<2, 0>(A, grp.ops, grid, after, grp.narrow, bs); break;
+                case 5: launch_batch<2, 1>(A, grp.ops, grid, after, grp.narrow, bs); break;
+                case 6: launch_batch<3, 0>(A, grp.ops, grid, after, grp.narrow, bs); break;
+                case 7: launch_batch<3, 1>(A, grp.ops, grid, after, grp.narrow, bs); break;
+                case 8: launch_batch<4, 0>(A, grp.ops, grid, after, grp.narrow, bs); break;
+                case 9: launch_batch<4, 1>(A, grp.ops, grid, after, grp.narrow, bs); break;
+                case 10: launch_batch<5, 0>(A, grp.ops, grid, after, grp.narrow, bs); break;
+                case 11: launch_batch<5, 1>(A, grp.ops, grid, after, grp.narrow, bs); break;
+                case 12: launch_batch<6, 0>(A, grp.ops, grid, after, grp.narrow, bs); break;
+                case 13: launch_batch<6, 1>(A, grp.ops, grid, after, grp.narrow, bs); break;
                 }
                 DGB_CUDA(cudaGetLastError());
                 launches++;

@@ -98,6 +98,7 @@ struct Batch {
     struct Group {
         int K = 0, begin = 0, end = 0;  // tiles[begin .. end)
         BatchOps ops{};
+        bool narrow = true;  // every problem's fields take 32-bit indices
     };
     std::vector<Group> groups;
     int counter_groups = 0;  // groups d_counters has room for

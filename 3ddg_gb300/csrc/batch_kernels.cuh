@@ -45,11 +45,19 @@ __device__ __forceinline__ void batch_exterior(const BatchProblem& P, int face, 
     }
 }
 
-template <int K, bool PDL>
-__device__ __forceinline__ float batch_in(const BatchProblem& P, const float* ub, const float* inc, int f, size_t off)
+// Off: the type of an index into a problem's fields, unsigned where all four
+// fields of a state have fewer than 2^32 values (batch_narrow): an index is one
+// multiply-add and an address one more, instead of two each, and the stage
+// phase spills nowhere (256 uneven problems 6717 -> 6254 us per step, 24 of them
+// 555 -> 529).
+inline bool batch_narrow(size_t fs) { return 4 * fs < ((size_t)1 << 32); }
+
+template <int K, bool PDL, typename Off>
+__device__ __forceinline__ float batch_in(const BatchProblem& P, const float* ub, const float* inc, int f, Off off)
 {
-    float v = pdl_load<PDL>(ub + (size_t)f * P.fs + off);
-    if (inc) v += pdl_load<PDL>(inc + (size_t)f * P.fs + off);
+    const Off o = (Off)f * (Off)P.fs + off;
+    float v = pdl_load<PDL>(ub + o);
+    if (inc) v += pdl_load<PDL>(inc + o);
     return v;
 }
 
@@ -140,7 +148,7 @@ struct BatchGradSmem {
 // to the buffer the pass before last read, which every owner finished before
 // the previous pass's barrier.  The owners' face-table codes of each pass
 // are loaded during the pass before.
-template <int K, bool PDL>
+template <int K, bool PDL, typename Off>
 __device__ void batch_grad_tile(const BatchProblem& P, const BatchOps& ops, const BatchTile& T, int stage,
                                 bool wait, unsigned char* smraw)
 {
@@ -168,14 +176,14 @@ __device__ void batch_grad_tile(const BatchProblem& P, const BatchOps& ops, cons
         batch_end_codes<K>(P, T, c0 + EPB, task, ls, a, code_next);
         // every other global load is issued before the first use
         float rho = 0.f;
-        if (act) rho = batch_in<K, PDL>(P, ub, inc, 0, (size_t)e * P.np + n);
+        if (act) rho = batch_in<K, PDL, Off>(P, ub, inc, 0, (Off)e * P.np + n);
         float ro[2] = {0.f, 0.f};
         if (owner) {
 #pragma unroll
             for (int side = 0; side < 2; side++) {
                 if (code[side] >= 0) {
-                    const size_t o2 = (size_t)code[side] * P.np + b0 + (side ? 0 : (K - 1) * st);
-                    ro[side] = batch_in<K, PDL>(P, ub, inc, 0, o2);
+                    const Off o2 = (Off)code[side] * P.np + b0 + (side ? 0 : (K - 1) * st);
+                    ro[side] = batch_in<K, PDL, Off>(P, ub, inc, 0, o2);
                 } else {
                     float uo;
                     batch_exterior(P, -1 - code[side], stage, ro[side], uo);
@@ -186,7 +194,7 @@ __device__ void batch_grad_tile(const BatchProblem& P, const BatchOps& ops, cons
         __syncthreads();
         if (owner) {
             const float* r = SM[ls].r[buf];
-            float* q = P.q + (size_t)a * P.fs + (size_t)(c0 + ls) * P.np;
+            float* q = P.q + ((Off)a * (Off)P.fs + (Off)(c0 + ls) * P.np);
             float v[K];
 #pragma unroll
             for (int j = 0; j < K; j++) v[j] = r[b0 + j * st];
@@ -205,7 +213,7 @@ __device__ void batch_grad_tile(const BatchProblem& P, const BatchOps& ops, cons
     }
 }
 
-template <int K, bool PDL>
+template <int K, bool PDL, typename Off>
 __device__ void batch_stage_tile(const BatchProblem& P, const BatchOps& ops, const BatchTile& T, int stage,
                                  bool wait, unsigned char* smraw)
 {
@@ -233,7 +241,7 @@ __device__ void batch_stage_tile(const BatchProblem& P, const BatchOps& ops, con
         const bool live = slot < EPB && e < T.e0 + T.count;
         const bool act = live && n < K3;
         PlainSmem<float, K>& S = SM[slot < EPB ? slot : 0];
-        const size_t off = (size_t)e * P.np + n;
+        const Off off = (Off)e * P.np + n, fs = (Off)P.fs;
         int code[R];
 #pragma unroll
         for (int r = 0; r < R; r++) code[r] = code_next[r];
@@ -249,12 +257,12 @@ __device__ void batch_stage_tile(const BatchProblem& P, const BatchOps& ops, con
         if (act) {
 #pragma unroll
             for (int f = 0; f < 4; f++) {
-                ubv[f] = pdl_load<PDL>(ub + (size_t)f * P.fs + off);
-                if (inc) dv[f] = pdl_load<PDL>(inc + (size_t)f * P.fs + off);
-                if (final_stage) cmp[f] = P.comp[(size_t)f * P.fs + off];
+                ubv[f] = pdl_load<PDL>(ub + (f * fs + off));
+                if (inc) dv[f] = pdl_load<PDL>(inc + (f * fs + off));
+                if (final_stage) cmp[f] = P.comp[f * fs + off];
             }
 #pragma unroll
-            for (int a = 0; a < 3; a++) q[a] = pdl_load<PDL>(P.q + (size_t)a * P.fs + off);
+            for (int a = 0; a < 3; a++) q[a] = pdl_load<PDL>(P.q + (a * fs + off));
         }
         float ro[R], uo[R], qo[R];
 #pragma unroll
@@ -264,10 +272,10 @@ __device__ void batch_stage_tile(const BatchProblem& P, const BatchOps& ops, con
             if (!live || t >= NF) continue;
             const FaceNodeArith<K> F(t);
             if (code[r] >= 0) {
-                const size_t o2 = (size_t)code[r] * P.np + F.nn;
-                ro[r] = batch_in<K, PDL>(P, ub, inc, 0, o2);
-                uo[r] = batch_in<K, PDL>(P, ub, inc, 1 + F.a, o2);
-                qo[r] = pdl_load<PDL>(P.q + (size_t)F.a * P.fs + o2);
+                const Off o2 = (Off)code[r] * P.np + F.nn;
+                ro[r] = batch_in<K, PDL, Off>(P, ub, inc, 0, o2);
+                uo[r] = batch_in<K, PDL, Off>(P, ub, inc, 1 + F.a, o2);
+                qo[r] = pdl_load<PDL>(P.q + (F.a * fs + o2));
             } else {
                 batch_exterior(P, -1 - code[r], stage, ro[r], uo[r]);
             }
@@ -365,7 +373,7 @@ __device__ void batch_stage_tile(const BatchProblem& P, const BatchOps& ops, con
             const float r[4] = {r_rho, r_u[0], r_u[1], r_u[2]};
 #pragma unroll
             for (int f = 0; f < 4; f++) {
-                const size_t o = (size_t)f * P.fs + off;
+                const Off o = f * fs + off;
                 float d = ca * r[f] + ubv[f] * ce;
                 if (inc) d += dv[f] * cbe;
                 if (final_stage) {
@@ -404,7 +412,9 @@ constexpr int BATCH_GRAD_BLOCKS = 8;
 // for K = 6: 123.3 G, against 121.9 G with 6 CTAs at 48 registers and
 // 121.5 G with 256-thread CTAs (with both phases in one kernel); with the
 // phases apart, the K = 6 update at 48 registers (6 CTAs, 4 bytes of spills)
-// measured 134.8 against 135.2 G.
+// measured 134.8 against 135.2 G.  With 32-bit indices: 5 CTAs at K = 5 6444, at
+// K = 3 6285, 6 at K = 6 6629, at K = 4 6251 against 6254 us per step.  A launch
+// with a block for every tile (PDL) has room for 80 registers (no spills).
 __host__ __device__ constexpr int batch_min_blocks(int K, int phase)
 {
     return phase == 0 ? BATCH_GRAD_BLOCKS : (K == 2 || K == 4 || K == 6 ? 5 : 4);
@@ -424,8 +434,8 @@ __device__ __forceinline__ void load_problem(BatchProblem& dst, const BatchProbl
 // step without any kernel waiting on another's blocks, and separate kernels,
 // so that each gets its own register budget.  A persistent grid pulls the
 // group's tiles from an atomic counter.
-template <int K, int PHASE, bool PDL>
-__global__ void __launch_bounds__(bthreads_of(K), batch_min_blocks(K, PHASE))
+template <int K, int PHASE, bool PDL, typename Off>
+__global__ void __launch_bounds__(bthreads_of(K), PDL && PHASE == 1 ? 3 : batch_min_blocks(K, PHASE))
     batch_stage_kernel(BatchArgs A, const BatchOps ops)
 {
     __shared__ __align__(16) unsigned char smraw[batch_smem_bytes<K, PHASE>()];
@@ -440,8 +450,8 @@ __global__ void __launch_bounds__(bthreads_of(K), batch_min_blocks(K, PHASE))
         // tiles, counters, descriptors and face tables are the same for all
         // kernels of a step: the wait for the kernel before comes after them
         if (P.active) {
-            if constexpr (PHASE == 0) batch_grad_tile<K, PDL>(P, ops, T, A.stage, first, smraw);
-            else batch_stage_tile<K, PDL>(P, ops, T, A.stage, first, smraw);
+            if constexpr (PHASE == 0) batch_grad_tile<K, PDL, Off>(P, ops, T, A.stage, first, smraw);
+            else batch_stage_tile<K, PDL, Off>(P, ops, T, A.stage, first, smraw);
             first = false;
         }
         if (A.n_tiles <= gridDim.x) break;

@@ -160,9 +160,14 @@ void launch_grad(Solver& s, const StageIO<T>& io, const MeshDev<T>& md)
     if constexpr (sizeof(T) == 4) {
         const int grid = (md.n_elem + incr_epb(K) - 1) / incr_epb(K);
         if (s.short_launches())
-            launch_pdl(incr_gradient_kernel<K, true>, grid, incr_threads(K), s.stream, io, md, host_const<T, K>(s, 3));
+            launch_pdl(incr_gradient_kernel<K, true, unsigned>, grid, incr_threads(K), s.stream, io, md,
+                       host_const<T, K>(s, 3));
+        else if (incr_narrow(io.fs))
+            incr_gradient_kernel<K, false, unsigned><<<grid, incr_threads(K), 0, s.stream>>>(io, md,
+                                                                                            host_const<T, K>(s, 3));
         else
-            incr_gradient_kernel<K, false><<<grid, incr_threads(K), 0, s.stream>>>(io, md, host_const<T, K>(s, 3));
+            incr_gradient_kernel<K, false, size_t><<<grid, incr_threads(K), 0, s.stream>>>(io, md,
+                                                                                          host_const<T, K>(s, 3));
     } else if (s.fix_ok[3]) {
         launch_pdl(ldg_gradient_fix_kernel<K>, (md.n_elem + fix_epb(K) - 1) / fix_epb(K), fix_threads(K), s.stream, io,
                    md, host_const<T, K>(s, 3), fix_set<K>(s).grad);
@@ -206,23 +211,23 @@ void launch_plain(const Solver& s, int slot, const StageIO<double>& io, const Me
     }
 }
 
-template <int K, bool DIFF, bool PDL>
+template <int K, bool DIFF, bool PDL, typename Off>
 constexpr auto incr_stage()
 {
-    if constexpr (incr_epb(K) > 1) return incr_packed_stage_kernel<K, DIFF, PDL>;
-    else return incr_stage_kernel<K, DIFF, PDL>;
+    if constexpr (incr_epb(K) > 1) return incr_packed_stage_kernel<K, DIFF, PDL, Off>;
+    else return incr_stage_kernel<K, DIFF, PDL, Off>;
 }
 
 template <int K, bool DIFF>
 void launch_incr(const Solver& s, const StageIO<float>& io, const MeshDev<float>& md, const OpConst<float, K>& C)
 {
-    const int grid = (md.n_elem + incr_epb(K) - 1) / incr_epb(K);
+    const int grid = (md.n_elem + incr_epb(K) - 1) / incr_epb(K), adv = s.p.eval_advect, sponge = s.p.eval_sponge;
     if (s.short_launches())
-        launch_pdl(incr_stage<K, DIFF, true>(), grid, incr_threads(K), s.stream, io, md, C, s.p.eval_advect,
-                   s.p.eval_sponge);
+        launch_pdl(incr_stage<K, DIFF, true, unsigned>(), grid, incr_threads(K), s.stream, io, md, C, adv, sponge);
+    else if (incr_narrow(io.fs))
+        incr_stage<K, DIFF, false, unsigned>()<<<grid, incr_threads(K), 0, s.stream>>>(io, md, C, adv, sponge);
     else
-        incr_stage<K, DIFF, false>()<<<grid, incr_threads(K), 0, s.stream>>>(io, md, C, s.p.eval_advect,
-                                                                              s.p.eval_sponge);
+        incr_stage<K, DIFF, false, size_t>()<<<grid, incr_threads(K), 0, s.stream>>>(io, md, C, adv, sponge);
 }
 
 template <typename T, int K>
