@@ -169,12 +169,6 @@ class ClockSampler:
 
 
 # ---------------------------------------------------------------- helpers
-# Orders N whose FP64 stage / gradient kernels use even-odd line owners (K = N + 1;
-# eo_lines and eo_grad_lines in 3ddg_gb300/csrc/dg_kernels.cuh), for the kernel labels.
-EO_STAGE_ORDERS = (1, 2, 4)
-EO_GRAD_ORDERS = (1, 2, 3, 4)
-
-
 def measured_peaks():
     p = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(p):
@@ -417,10 +411,9 @@ def run_ours(a, dist: Dist):
     roof = {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": (ach / peak) if ach else None,
             "traffic": traffic, "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured"
             else "fallback 6.8 TB/s",
-            "kernel": (("stage_kernel<double,%d,DIFF,2,EO> (fluxes read, even-odd line owners)" % (cfg["ORDER"] + 1)
-                        if cfg["ORDER"] in EO_STAGE_ORDERS
-                        else "stage_kernel<double,%d,DIFF,2> (fluxes read, per-node line sums)" % (cfg["ORDER"] + 1))
-                       if fp64 else "incr_stage_kernel<float,%d,DIFF>" % (cfg["ORDER"] + 1)),
+            "kernel": ("stage_fix_kernel<%d,DIFF,2> (fluxes read, fixed-point line operators)" % (cfg["ORDER"] + 1)
+                       if fp64 else "incr_%sstage_kernel<%d,DIFF>" % ("packed_" if cfg["ORDER"] <= 3 else "",
+                                                                       cfg["ORDER"] + 1)),
             "algorithmic_bytes_per_launch": st_b / st_n if st_n else None,
             "traffic_note": ("above the algorithmic bytes by the volume-flux buffers (4 values written and 4 read "
                              "per node, 64 B): HBM traded for the FP64 work of evaluating each face neighbour's "
@@ -429,14 +422,12 @@ def run_ours(a, dist: Dist):
             "fp64_pipe": {"achieved_tflops": (st_f / st_n) / (st_ms / st_n / 1e3) / 1e12 if st_n else None,
                           "peak_tflops": FP64_PEAK_TFLOPS,
                           "frac": ((st_f / st_n) / (st_ms / st_n / 1e3) / 1e12) / FP64_PEAK_TFLOPS if st_n else None,
-                          "note": "the FP64 path is bound by the FP64 pipe (1.19 TFLOP/s measured), not HBM; "
-                                  "flops counted by the direct formula (K (K + 2) per line), which the even-odd "
-                                  "line owners execute with about 22 % fewer FP64 instructions"},
+                          "note": "flops counted by the direct formula (K (K + 2) per line); the line sums run as "
+                                  "block fixed point on the integer pipes, so that this exceeds the FP64 pipe's "
+                                  "1.19 TFLOP/s; 12 to 16 operations per node and stage are left on that pipe"},
             "share_of_step": st_ms / ms if ms else None,
-            "gradient_kernel": {"name": ("ldg_gradient_eo_kernel<%d>" % (cfg["ORDER"] + 1)
-                                         if fp64 and cfg["ORDER"] in EO_GRAD_ORDERS else
-                                         ("ldg_gradient_kernel<double,%d>" if fp64 else "ldg_gradient_kernel<float,%d>")
-                                         % (cfg["ORDER"] + 1)),
+            "gradient_kernel": {"name": ("ldg_gradient_fix_kernel<%d>" if fp64 else "incr_gradient_kernel<%d>")
+                                % (cfg["ORDER"] + 1),
                                 "launches": gr_n, "mean_launch_ms": gr_ms / gr_n if gr_n else None,
                                 "achieved_gbs": (gr_b / gr_n) / (gr_ms / gr_n / 1e3) / 1e9 if gr_n else None}}
     line = {
