@@ -71,20 +71,17 @@ void fill_ops(BatchProblem& P, const LineOperators& op, const dg_params& p)
     P.linear_mass = C.linear_mass;
 }
 
-// A launch with a block for every tile starts under the one before it in its
-// branch (launch_pdl; with the step bookkeeping in one launch, 8 problems of
-// 4..8 elements per axis 53 -> 42 us per step, one of 6^3 32 -> 20 us); one
-// whose blocks stream several has no gap to hide and keeps the read-only loads
-// and the smaller register budget (24 uneven problems, about two tiles per
-// block: 581 us per step when launched so, 529 when not).  The first launch of
-// a step (``after`` false) reads descriptors that the launch before it wrote,
-// so it waits for it.
+// ``dependent``: the launch starts under the one before it in its branch
+// (launch_pdl).  That takes a block for every tile; a launch whose blocks stream
+// several has no gap to hide and keeps the read-only loads and the smaller
+// register budget (24 uneven problems, about two tiles per block: 581 us per
+// step when launched so, 529 when not).
 template <int K, int PHASE>
-void launch_batch(const BatchArgs& A, const BatchOps& ops, int grid, bool after, bool narrow, cudaStream_t st)
+void launch_batch(const BatchArgs& A, const BatchOps& ops, int grid, bool dependent, bool narrow, cudaStream_t st)
 {
     if (!narrow)
         batch_stage_kernel<K, PHASE, false, size_t><<<grid, bthreads_of(K), 0, st>>>(A, ops);
-    else if (after && A.n_tiles <= grid)
+    else if (dependent && A.n_tiles <= grid)
         launch_pdl(batch_stage_kernel<K, PHASE, true, unsigned>, grid, bthreads_of(K), st, A, ops);
     else
         batch_stage_kernel<K, PHASE, false, unsigned><<<grid, bthreads_of(K), 0, st>>>(A, ops);
@@ -552,6 +549,15 @@ int Batch::launch_step()
     const int nb = G > 1 ? std::min(G, (int)kBranches) : 0;
     if (nb) DGB_CUDA(cudaEventRecord(fork_ev, stream));
     for (int b = 0; b < nb; b++) DGB_CUDA(cudaStreamWaitEvent(branch[b], fork_ev, 0));
+    // Dependent launches only while the step's tiles all fit on the device at once:
+    // blocks that wait for their predecessor hold slots that the other branches
+    // could use.  8 problems of 4..8 elements per axis (933 tiles) 45.7 us per
+    // step without, 43.1 with; one of 6^3 (54) 24.3, 19.6; a served mix of
+    // 1300 to 2800 tiles 33.8 ms of device time without, 35.6 with (and its
+    // graph, whose edges then change with the tile counts, is instantiated anew).
+    int tiles_all = 0;
+    for (const Group& grp : groups) tiles_all += grp.end - grp.begin;
+    const bool small = tiles_all <= num_sms * BATCH_GRAD_BLOCKS;
     for (int g = 0; g < G; g++) {
         const Group& grp = groups[g];
         const int K = grp.K;
@@ -569,18 +575,19 @@ int Batch::launch_step()
             for (int phase = 0; phase < 2; phase++) {
                 const int grid =
                     std::max(1, std::min(num_sms * std::min(ctas_per_sm, occ_k[K][phase]), A.n_tiles));
-                const bool after = s + phase > 0;
+                // the first launch reads descriptors that the launch before it wrote
+                const bool dependent = small && s + phase > 0;
                 switch (K * 2 + phase) {
-                case 4: launch_batch<2, 0>(A, grp.ops, grid, after, grp.narrow, bs); break;
-                case 5: launch_batch<2, 1>(A, grp.ops, grid, after, grp.narrow, bs); break;
-                case 6: launch_batch<3, 0>(A, grp.ops, grid, after, grp.narrow, bs); break;
-                case 7: launch_batch<3, 1>(A, grp.ops, grid, after, grp.narrow, bs); break;
-                case 8: launch_batch<4, 0>(A, grp.ops, grid, after, grp.narrow, bs); break;
-                case 9: launch_batch<4, 1>(A, grp.ops, grid, after, grp.narrow, bs); break;
-                case 10: launch_batch<5, 0>(A, grp.ops, grid, after, grp.narrow, bs); break;
-                case 11: launch_batch<5, 1>(A, grp.ops, grid, after, grp.narrow, bs); break;
-                case 12: launch_batch<6, 0>(A, grp.ops, grid, after, grp.narrow, bs); break;
-                case 13: launch_batch<6, 1>(A, grp.ops, grid, after, grp.narrow, bs); break;
+                case 4: launch_batch<2, 0>(A, grp.ops, grid, dependent, grp.narrow, bs); break;
+                case 5: launch_batch<2, 1>(A, grp.ops, grid, dependent, grp.narrow, bs); break;
+                case 6: launch_batch<3, 0>(A, grp.ops, grid, dependent, grp.narrow, bs); break;
+                case 7: launch_batch<3, 1>(A, grp.ops, grid, dependent, grp.narrow, bs); break;
+                case 8: launch_batch<4, 0>(A, grp.ops, grid, dependent, grp.narrow, bs); break;
+                case 9: launch_batch<4, 1>(A, grp.ops, grid, dependent, grp.narrow, bs); break;
+                case 10: launch_batch<5, 0>(A, grp.ops, grid, dependent, grp.narrow, bs); break;
+                case 11: launch_batch<5, 1>(A, grp.ops, grid, dependent, grp.narrow, bs); break;
+                case 12: launch_batch<6, 0>(A, grp.ops, grid, dependent, grp.narrow, bs); break;
+                case 13: launch_batch<6, 1>(A, grp.ops, grid, dependent, grp.narrow, bs); break;
                 }
                 DGB_CUDA(cudaGetLastError());
                 launches++;
