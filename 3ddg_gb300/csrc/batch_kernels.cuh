@@ -9,18 +9,15 @@
 // RK stage each group gets two launches of a persistent kernel of its order
 // (batch_stage_kernel<K>, K = N + 1 <= 6) that take tiles (problem, first
 // element, element count), the first by block number, the rest from an atomic
-// counter: the LDG gradient of every
-// tile, then the stage update of every tile, with EPB(K) elements per pass of
-// a CTA of bthreads_of(K) threads; the number of passes per tile (tile size) is chosen per
-// order by the autotuner.  Groups run as parallel branches of the step.  The
-// arithmetic per element is the one of incr_stage_kernel /
-// ldg_gradient_kernel (dg_kernels.cuh) with 1/w_a applied after the line
-// sums, so one descriptor serves all three stages and the group's operator
+// counter: the LDG gradient of every tile, then the stage update of every tile,
+// with EPB(K) elements per pass of a CTA of bthreads_of(K) threads; the number
+// of passes per tile (tile size) is chosen per order by the autotuner.  Groups
+// run as parallel branches of the step.  The arithmetic per element is the one
+// of incr_kernels.cuh with 1/w_a applied after the line sums, so one descriptor serves all three stages and the group's operator
 // rows (kernel parameters) do not depend on the axis.  Face nodes are decoded
-// arithmetically (FaceNodeArith): the table lookup the single-problem kernels
-// use measured 2 % slower here (115.1 vs 117.3 G on config 4).
+// arithmetically (FaceNodeArith): a table lookup measured 2 % slower here
+// (115.1 vs 117.3 G on config 4).
 #pragma once
-
 
 #include "batch_types.h"
 #include "dg_kernels.cuh"

@@ -344,10 +344,10 @@ __device__ __forceinline__ void stage_fix_line(const OpConst<double, K>& C, cons
 // What bounds these kernels and what they measured (ms per launch at 32.8 M
 // nodes, even-odd or per-node FP64 line sums -> fixed point):
 //   K          2           3           4           5           6           7           8
-//   stage      8.99->1.44  4.49->1.43  3.85->1.21  3.85->1.35  4.28->1.47  4.69->1.67  5.67->1.56
-//   gradient   1.54->0.57  1.10->0.42  1.11->0.43  1.11->0.41  1.40->0.52  1.60->0.53  1.69->0.54
-// At K = 5 a stage launch keeps the FP64 pipe about 62 % busy (16 operations per
-// node), the integer pipe 50 %, the issue slots 60 % and HBM at 65 % of a copy:
+//   stage      8.99->1.40  4.49->1.41  3.85->1.18  3.85->1.32  4.28->1.41  4.69->1.66  5.67->1.51
+//   gradient   1.54->0.55  1.10->0.41  1.11->0.41  1.11->0.38  1.40->0.49  1.60->0.51  1.69->0.52
+// At K = 5 a stage launch keeps the FP64 pipe 69 % busy (16 operations per
+// node), the integer pipe 53 %, the issue slots 62 % and HBM at 71 % of a copy:
 // no unit is the bound by itself, the barriers between the node and line phases
 // are (26 % of the warps' time), so resident warps count most.  Registers per
 // thread of the stage kernel and elements per CTA were chosen by that (us per

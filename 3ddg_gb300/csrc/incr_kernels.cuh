@@ -1,7 +1,7 @@
 // FP32 kernels of one RK stage (increment form): the LDG gradient and the
 // stage update.  Bound by issue, the L1 data pipe and the latency of the global
-// loads, not by arithmetic (64^3 elements at N = 4: issue slots 55-70 % busy,
-// L1 wavefronts 51-65 %, HBM 54-60 %).
+// loads, not by arithmetic (64^3 elements at N = 4, stage kernel: issue
+// slots 68 % busy, L1 wavefronts 58 %, HBM 55 %).
 //
 // Mapping: a CTA takes incr_epb(K) whole elements.  Thread t has node t of
 // their nodes, packed densely; the lines of one axis, packed over the elements,
@@ -20,6 +20,8 @@
 //   K = 2  497 / 191 -> 184 / 81    K = 5 (32.8 M nodes)  532 / 230 -> 542 / 217
 //   K = 3  236 / 100 -> 165 / 69    K = 7                 161 / 69  -> 161 / 62
 //   K = 4  177 /  81 -> 134 / 59    K = 8                 192 / 70  -> 172 / 59
+// and with 32-bit field offsets (incr_at), ~32.8 M nodes, K = 2 .. 8:
+//   714 / 305, 646 / 259, 511 / 220, 506 / 213, 625 / 227, 631 / 253, 690 / 220
 #pragma once
 
 #include "dg_kernels.cuh"
