@@ -227,64 +227,39 @@ struct FixSmem {
     double q[3][fix_slots(K)];
 };
 
-// The line in FP64, for values fixed point cannot hold (and lines of zeros),
-// with axis 0's operator like the fixed-point form.
-template <int K, bool DIFF>
-__device__ __noinline__ void stage_line_fp64(const OpConst<double, K>& C, FixSmem<K>& S, int a, int sb0, int sst,
-                                             double fmo0, double fmoN, double fao0, double faoN, double qo0,
-                                             double qoN)
+// One equation of a line in FP64, for values fixed point cannot hold (and lines
+// of zeros), with axis 0's operator like the fixed-point form: v (+ w) at the
+// line's nodes, g its lift-scaled face fluxes.
+template <int K>
+__device__ __noinline__ void stage_line_fp64(const OpConst<double, K>& C, const double* pv, const double* pw, int sst,
+                                             double g0, double gN, double* out)
 {
-    double gm[2], gr[2], v[K];
-    long long any = fix_bits(fmo0) | fix_bits(fmoN) | fix_bits(fao0) | fix_bits(faoN) | fix_bits(qo0) | fix_bits(qoN);
-#pragma unroll 1
+    double v[K];
+    long long any = fix_bits(g0) | fix_bits(gN);
+#pragma unroll
     for (int j = 0; j < K; j++) {
-        const int o = sb0 + j * sst;
-        any |= fix_bits(S.fm[o]) | fix_bits(S.fa[a][o]);
-        if (DIFF) any |= fix_bits(S.q[a][o]);
+        v[j] = pv[j * sst];
+        any |= fix_bits(v[j]);
+        if (pw) {
+            any |= fix_bits(pw[j * sst]);
+            v[j] += pw[j * sst];
+        }
     }
     if (any << 1 == 0) {  // +-0 everywhere
 #pragma unroll 1
-        for (int j = 0; j < K; j++) S.fa[a][sb0 + j * sst] = S.q[a][sb0 + j * sst] = 0.0;
+        for (int j = 0; j < K; j++) out[j * sst] = 0.0;
         return;
     }
 #pragma unroll 1
-    for (int side = 0; side < 2; side++) {
-        const int o = sb0 + (side ? (K - 1) * sst : 0);
-        const double fmo = side ? fmoN : fmo0, fao = side ? faoN : fao0;
-        const double* cm = C.cM[0][side];
-        const double* cr = C.cA[0][side];
-        gm[side] = fmo * cm[0] + S.fm[o] * cm[1] + fao * cm[2] + S.fa[a][o] * cm[3];
-        gr[side] = fmo * cr[0] + S.fm[o] * cr[1] + fao * cr[2] + S.fa[a][o] * cr[3];
-        if (DIFF) gr[side] += C.cQ[0][side] * ((side ? qoN : qo0) + S.q[a][o]);
-    }
-#pragma unroll
-    for (int j = 0; j < K; j++) {
-        const int o = sb0 + j * sst;
-        v[j] = DIFF ? S.fa[a][o] + S.q[a][o] : S.fa[a][o];
-    }
-#pragma unroll 1
     for (int i = 0; i < K; i++) {
         const double* row = C.rows[0][i];
-        double s = row[K] * gr[0];
-        s += row[K + 1] * gr[1];
+        double s = row[K] * g0;
+        s += row[K + 1] * gN;
 #pragma unroll
         for (int j = 0; j < K; j++) s += row[j] * v[j];
-        S.fa[a][sb0 + i * sst] = s;
-    }
-#pragma unroll
-    for (int j = 0; j < K; j++) v[j] = S.fm[sb0 + j * sst];
-#pragma unroll 1
-    for (int i = 0; i < K; i++) {
-        const double* row = C.rows[0][i];
-        double s = row[K] * gm[0];
-        s += row[K + 1] * gm[1];
-#pragma unroll
-        for (int j = 0; j < K; j++) s += row[j] * v[j];
-        S.q[a][sb0 + i * sst] = s;
+        out[i * sst] = s;
     }
 }
-
-__device__ __forceinline__ int high_word(const double* p) { return reinterpret_cast<const int*>(p)[1]; }
 
 // One line of the stage: the mass equation's sums (of f_mass + G and its face
 // terms) into S.fa[a], the momentum equation's into S.q[a].  With the face
@@ -292,52 +267,38 @@ __device__ __forceinline__ int high_word(const double* p) { return reinterpret_c
 // left and -x X + y Y at the right end (FixLine), with
 //   momentum  X = f_mom' + f_mom,              Y = f_mass' - f_mass
 //   mass      X = f_mass' + f_mass + G' + G,   Y = f_mom' - f_mom
-// (' across the face): sums of fixed-point values, exact.
+// (' across the face): the sums are exact in fixed point, the differences FP64.
 template <int K, bool DIFF>
-__device__ __forceinline__ void stage_fix_line(const OpConst<double, K>& C, const FixLine<K, 2>& L,
-                                               int pm, FixSmem<K>& S, int a, int sb0, int sst, const double fmo[2],
-                                               const double fao[2], const double qo[2], int do_adv)
+__device__ __forceinline__ void stage_fix_line(const OpConst<double, K>& C, const FixLine<K, 2>& L, int pm,
+                                               FixSmem<K>& S, int a, int sb0, int sst, const double (&fmo)[2],
+                                               const double (&fao)[2], const double (&qo)[2], int do_adv)
 {
-    // exponent of the line: the high words only, so that no value is held
-    // while the others are read
-    int tm = max(fix_abs_hi(fmo[0]), fix_abs_hi(fmo[1])), ta = max(fix_abs_hi(fao[0]), fix_abs_hi(fao[1]));
-    if (DIFF) ta = max(ta, max(fix_abs_hi(qo[0]), fix_abs_hi(qo[1])));
-#pragma unroll
-    for (int j = 0; j < K; j++) {
-        const int o = sb0 + j * sst;
-        tm = max(tm, high_word(&S.fm[o]) & 0x7fffffff);
-        ta = max(ta, high_word(&S.fa[a][o]) & 0x7fffffff);
-        if (DIFF) ta = max(ta, high_word(&S.q[a][o]) & 0x7fffffff);
-    }
-    const int E = max((tm >> 20) + pm, ta >> 20), Em = E - pm;
-    if (E < kFixMinExp || E > kFixMaxExp) {
-        stage_line_fp64<K, DIFF>(C, S, a, sb0, sst, fmo[0], fmo[1], fao[0], fao[1], qo[0], qo[1]);
-        return;
-    }
     const int sN = sb0 + (K - 1) * sst;
-    FixVal x[K];
-    const FixVal m0 = fix_from(fmo[0], Em), mN = fix_from(fmo[1], Em);
-    const FixVal s0 = fix_from(S.fm[sb0], Em), sn = fix_from(S.fm[sN], Em);
-    FixVal C0 = fix_from(fao[0], E), CN = fix_from(fao[1], E);
-#pragma unroll
-    for (int j = 0; j < K; j++) x[j] = fix_from(S.fa[a][sb0 + j * sst], E);
-    const FixVal B0 = C0 - x[0], BN = CN - x[K - 1];
-    if (DIFF) {
-        C0 = C0 + fix_from(qo[0], E);
-        CN = CN + fix_from(qo[1], E);
-#pragma unroll
-        for (int j = 0; j < K; j++) x[j] = x[j] + fix_from(S.q[a][sb0 + j * sst], E);
-    }
+    double* fm = &S.fm[sb0];
     double* fa = &S.fa[a][sb0];
-    const int er = E + L.e_out[1];
-    fix_line<K, 2>(L, 1, x, C0 + x[0], CN + x[K - 1], m0 - s0, mN - sn,
-                   [&](int i, long long o) { fa[i * sst] = fix_to(o, er); });
-    if (do_adv) {
+    double* q = &S.q[a][sb0];
+    const double ya0 = fmo[0] - S.fm[sb0], yaN = fmo[1] - S.fm[sN];
+    // before the mass results replace f_mass
+    const double ym0 = fao[0] - S.fa[a][sb0], ymN = fao[1] - S.fa[a][sN];
+    if (!fix_equation<K, DIFF>(L, 1, -pm, fa, q, sst, fao, qo, ya0, yaN, fa)) {
+        double g[2];
 #pragma unroll
-        for (int j = 0; j < K; j++) x[j] = j == 0 ? s0 : j == K - 1 ? sn : fix_from(S.fm[sb0 + j * sst], Em);
-        double* q = &S.q[a][sb0];
-        const int em = E + L.e_out[0];
-        fix_line<K, 2>(L, 0, x, m0 + s0, mN + sn, B0, BN, [&](int i, long long o) { q[i * sst] = fix_to(o, em); });
+        for (int s = 0; s < 2; s++) {
+            const double* c = C.cA[0][s];
+            const int o = s ? sN : sb0;
+            g[s] = (s ? yaN : ya0) * c[0] + fao[s] * c[2] + S.fa[a][o] * c[3];
+            if (DIFF) g[s] += C.cQ[0][s] * (qo[s] + S.q[a][o]);
+        }
+        stage_line_fp64<K>(C, fa, DIFF ? q : nullptr, sst, g[0], g[1], fa);
+    }
+    if (do_adv && !fix_equation<K, false>(L, 0, pm, fm, nullptr, sst, fmo, fmo, ym0, ymN, q)) {
+        double g[2];
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+            const double* c = C.cM[0][s];
+            g[s] = fmo[s] * c[0] + S.fm[s ? sN : sb0] * c[1] + (s ? ymN : ym0) * c[2];
+        }
+        stage_line_fp64<K>(C, fm, nullptr, sst, g[0], g[1], q);
     }
 }
 
@@ -346,16 +307,18 @@ __device__ __forceinline__ void stage_fix_line(const OpConst<double, K>& C, cons
 //   K          2           3           4           5           6           7           8
 //   stage      8.99->1.40  4.49->1.41  3.85->1.18  3.85->1.32  4.28->1.41  4.69->1.66  5.67->1.51
 //   gradient   1.54->0.55  1.10->0.41  1.11->0.41  1.11->0.38  1.40->0.49  1.60->0.51  1.69->0.52
-// At K = 5 a stage launch keeps the FP64 pipe 69 % busy (16 operations per
-// node), the integer pipe 53 %, the issue slots 62 % and HBM at 71 % of a copy:
+// (with one exponent for both equations of a line; fix_equation has the cost of
+// one each).  At K = 5 a stage launch kept the FP64 pipe 69 % busy (16 operations
+// per node), the integer pipe 53 %, the issue slots 62 % and HBM at 71 % of a copy:
 // no unit is the bound by itself, the barriers between the node and line phases
 // are (26 % of the warps' time), so resident warps count most.  Registers per
 // thread of the stage kernel and elements per CTA were chosen by that (us per
 // launch on 8 M nodes: K = 5 at 40 / 48 / 56 / 80 registers 335 / 329 / 358 /
 // 537; K = 8 at 32 / 40 / 48 380 / 404 / 494; K = 4 at 1 / 2 / 4 / 6 elements
-// 383 / 296 / 311 / 349).  Converting results on the FP64 pipe (fix_to_fp64)
+// 383 / 296 / 311 / 349; with an exponent per equation K = 2 at 48 / 56 / 64
+// registers 448 / 432 / 459, the other orders as before).  Converting results on the FP64 pipe (fix_to_fp64)
 // instead saves integer work where that pipe is the scarcer one: 346 for 329 us.
-__host__ __device__ constexpr int fix_regs(int K) { return K == 8 ? 32 : K == 6 ? 56 : 48; }
+__host__ __device__ constexpr int fix_regs(int K) { return K == 8 ? 32 : K == 6 || K == 2 ? 56 : 48; }
 __host__ __device__ constexpr int fix_min_blocks(int K) { return 65536 / (fix_regs(K) * fix_threads(K)); }
 // The stage input and the old state are fetched into shared memory at the
 // start where they fit beside the line data.
@@ -536,9 +499,7 @@ inline bool make_stage_fix(const OpConst<double, K>& C, FixOps<K, 2>& F)
     if (!(k > 0x1p-40 && k < 0x1p40)) return false;
     F.pm = (int)std::lround(std::log2(k));
     const FixFlux f[2] = {{x, y, F.pm}, {h, g, -F.pm}};
-    if (!fix_axis<K, 2>(C.rows[0], 1, f, F.line)) return false;
-    F.line.e_out[0] -= F.pm;
-    return true;
+    return fix_axis<K, 2>(C.rows[0], 1, f, F.line);
 }
 
 // The same of the gradient operator (its flux factors are in the lift

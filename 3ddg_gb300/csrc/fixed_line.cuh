@@ -243,6 +243,57 @@ __host__ __device__ __forceinline__ void fix_line(const FixLine<K, NEQ>& L, int 
 // Exponent fields of a line's largest value that fixed point takes.
 constexpr int kFixMinExp = 200, kFixMaxExp = 1900;
 
+__host__ __device__ __forceinline__ int fix_max(int a, int b) { return a > b ? a : b; }
+
+// fix_abs_hi of a value in memory, of which it reads the high word alone, so
+// that no value is held while a line's others are read.
+__host__ __device__ __forceinline__ int fix_abs_hi_at(const double* p)
+{
+#ifdef __CUDA_ARCH__
+    return reinterpret_cast<const int*>(p)[1] & 0x7fffffff;
+#else
+    return fix_abs_hi(*p);
+#endif
+}
+
+// One equation of a line: outputs out[i st] from the node values v[j st]
+// (+ w[j st] with TWO), their counterparts vo (+ wo) across the two ends and
+// the jumps y across them that enter with the factor 2^py (FixFlux).  v, w and
+// out may be the same memory.  The exponent is that of the largest of these
+// values alone: an equation's sums keep their bits however large the other
+// equation's fluxes are, of which it sees no more than the jumps, formed in
+// FP64.  (One exponent for both lost the smaller: at u = 3.3e-4 m/s-scale mass
+// fluxes and drho = 1e-8 the momentum sums were off by 5e-8 of their largest.)
+// False, and nothing written, when fixed point cannot hold the values.
+template <int K, bool TWO>
+__host__ __device__ __forceinline__ bool fix_equation(const FixLine<K, 2>& L, int eq, int py, const double* v,
+                                                      const double* w, int st, const double (&vo)[2],
+                                                      const double (&wo)[2], double y0, double yN, double* out)
+{
+    int t = fix_max(fix_abs_hi(vo[0]), fix_abs_hi(vo[1]));
+    if (TWO) t = fix_max(t, fix_max(fix_abs_hi(wo[0]), fix_abs_hi(wo[1])));
+#pragma unroll
+    for (int j = 0; j < K; j++) {
+        t = fix_max(t, fix_abs_hi_at(v + j * st));
+        if (TWO) t = fix_max(t, fix_abs_hi_at(w + j * st));
+    }
+    const int E = fix_max(t >> 20, (fix_max(fix_abs_hi(y0), fix_abs_hi(yN)) >> 20) - py);
+    if (E < kFixMinExp || E > kFixMaxExp) return false;
+    FixVal x[K], X0 = fix_from(vo[0], E), XN = fix_from(vo[1], E);
+#pragma unroll
+    for (int j = 0; j < K; j++) x[j] = fix_from(v[j * st], E);
+    if (TWO) {
+        X0 = X0 + fix_from(wo[0], E);
+        XN = XN + fix_from(wo[1], E);
+#pragma unroll
+        for (int j = 0; j < K; j++) x[j] = x[j] + fix_from(w[j * st], E);
+    }
+    const int eo = E + L.e_out[eq];
+    fix_line<K, 2>(L, eq, x, X0 + x[0], XN + x[K - 1], fix_from(y0, E + py), fix_from(yN, E + py),
+                   [&](int i, long long o) { out[i * st] = fix_to(o, eo); });
+    return true;
+}
+
 // ------------------------------------------------------------------ host
 // The operator from rows (D_i0..D_i,K-1, L0_i, LN_i) and, per equation, the
 // flux factors x, y (value x X + y Y at the left end, -x X + y Y at the right;

@@ -1,0 +1,147 @@
+"""Right-hand sides against extended-precision sums of the operator in use:
+states whose momentum and mass fluxes are of very different size, and operators
+from matrix files whose mirror symmetry is broken a little (the fixed-point
+kernels apply what row K-1-i has beyond the mirror image of row i) or more (the
+FP64 kernels of dg_kernels.cuh).
+
+Bound: with T the sum over axes of (largest operator row sum) x (largest value
+of the equation's own terms), a fixed-point sum is off by at most 131 of its
+units, 17 x 2^-53 T per axis, and a chain of K + 6 FP64 operations by at most
+14 x 2^-53 T; with the fluxes, the stage combination and LDG's two levels,
+64 x 2^-53 T.
+"""
+import ctypes as C
+import os
+
+import numpy as np
+import pytest
+
+from conftest import dg, max_rel, workloads
+
+pytestmark = pytest.mark.gpu
+
+q = np.longdouble
+EPS = 64 * 2.0 ** -53
+
+
+class Reference:
+    """The semi-discrete scheme of one block of ``ne`` elements in extended
+    precision, zero outside non-periodic faces, and per equation the T of the
+    bound above.  Numerical fluxes by the jumps of the other equation's flux."""
+
+    def __init__(self, cfg, ops):
+        self.cfg, self.K, self.ne = cfg, cfg["ORDER"] + 1, cfg["NUM_ELEMENTS"]
+        self.D, self.L0, self.LN = (ops[k].astype(q) for k in ("deriv", "lift0", "liftN"))
+        self.row = float(np.max(np.abs(self.D).sum(1) + np.abs(self.L0) + np.abs(self.LN)))
+
+    def split(self, g):
+        K, (X, Y, Z) = self.K, self.ne
+        return g.astype(q).reshape(-1, X, K, Y, K, Z, K).transpose(0, 1, 3, 5, 2, 4, 6)
+
+    def join(self, u):
+        K, (X, Y, Z) = self.K, self.ne
+        return u.transpose(0, 1, 4, 2, 5, 3, 6).reshape(-1, X * K, Y * K, Z * K)
+
+    def along(self, v, a):
+        return np.moveaxis(np.moveaxis(v, 3 + a, -1) @ self.D.T, -1, 3 + a)
+
+    def ends(self, v, a):
+        lo, hi = np.take(v, 0, axis=3 + a), np.take(v, self.K - 1, axis=3 + a)
+        left, right = np.roll(hi, 1, a), np.roll(lo, -1, a)
+        if not self.cfg["BC_IS_PERIODIC"][a]:
+            s = [slice(None)] * 5
+            s[a] = 0
+            left[tuple(s)] = 0
+            s[a] = self.ne[a] - 1
+            right[tuple(s)] = 0
+        return lo, hi, left, right
+
+    def lift(self, g0, gN, a):
+        shape = [1] * 6
+        shape[3 + a] = self.K
+        return self.L0.reshape(shape) * np.expand_dims(g0, 3 + a) + self.LN.reshape(shape) * np.expand_dims(gN, 3 + a)
+
+    def rhs(self, rho, vel, sigma):
+        c = self.cfg
+        c0, r0, ba, Dc = (q(c[k]) for k in ("C0", "RHO0", "B_OVER_A", "DIFF_CONST"))
+        u, sig = self.split(np.concatenate([rho[None], vel])), self.split(sigma[None])[0]
+        d = u[0]
+        size = [0.0, 0.0, 0.0, 0.0]
+        out = [np.zeros_like(d)]
+        fm = c0 * c0 / r0 * (d + ba / (2 * r0) * d * d)
+        for a in range(3):
+            w = q(c["ELEMENT_WIDTH"][a])
+            fa = u[1 + a] * (r0 if ba == 0 else d + r0)
+            m0, mN, ml, mr = self.ends(fm, a)
+            a0, aN, al, ar = self.ends(fa, a)
+            k, g = c0 / (2 * r0), r0 / (2 * c0)
+            out.append((self.along(fm, a) + self.lift((ml + m0) / 2 + k * (al - a0),
+                                                      -((mr + mN) / 2 + k * (aN - ar)), a)) / w)
+            f = self.along(fa, a) + self.lift((al + a0) / 2 + g * (ml - m0), -((ar + aN) / 2 + g * (mN - mr)), a)
+            most = lambda *v: max(float(np.max(np.abs(x))) for x in v)  # noqa: E731
+            size[1 + a] += self.row * most(fm, k * (al - a0), k * (aN - ar)) / float(w)
+            size[0] += self.row * most(fa, g * (ml - m0), g * (mN - mr)) / float(w)
+            if c["EVALUATE_DIFFUSION"]:
+                d0, dN, dl, dr = self.ends(d, a)
+                G = (self.along(d, a) + self.lift((dl + d0) / 2, -(dr + dN) / 2, a)) * (Dc / w)
+                q0, qN, ql, qr = self.ends(G, a)
+                f = f + self.along(G, a) + self.lift((ql + q0) / 2, -(qr + qN) / 2, a)
+                size[0] += self.row * most(G) / float(w)
+                size[0] += self.row * self.row * float(Dc) * most(d) / float(w) ** 2
+            out[0] = out[0] + f / w
+        top = float(np.max(np.abs(sig)))
+        size = [s + top * float(np.max(np.abs(u[i]))) for i, s in enumerate(size)]
+        return self.join(np.stack(out) - sig * u), size
+
+
+def problem(order, ne=(3, 2, 4), periodic=(0, 0, 0), **kw):
+    cfg = workloads().gaussian_pulse(seed=5, num_elements=ne, order=order, width=0.5, sponge=1, periodic=periodic, **kw)
+    cfg["DT"] = workloads().cfl_dt(cfg)
+    return cfg
+
+
+def acoustic_state(dims, seed):
+    rng = np.random.default_rng(seed)
+    return rng.standard_normal(dims) * 1e-3, rng.standard_normal((3,) + tuple(dims)) * 1e-6
+
+
+def check(cfg, ops, s, rho, vel, fields=range(4)):
+    _, sigma = s.grid()
+    s.set_state(rho, vel)
+    r, v = s.rhs()
+    want, size = Reference(cfg, ops).rhs(rho, vel, sigma)
+    got = np.concatenate([r[None], v])
+    for f in fields:
+        err = float(np.max(np.abs(got[f].astype(q) - want[f])))
+        assert err <= EPS * size[f], (f, err / size[f])
+
+
+# ----------------------------------------------------- fluxes of uneven size
+@pytest.mark.parametrize("order", [1, 2, 3, 4, 5, 6, 7])
+@pytest.mark.parametrize("size", [1e-4, 1e-8, 1e-12, 1e-18])
+def test_momentum_of_small_densities_beside_large_velocities(order, size):
+    """A uniform flow that carries a density disturbance far below a sound
+    wave's: the momentum equation sees the disturbance alone (linear fluxes:
+    the mass flux has no jumps) and keeps its precision."""
+    cfg = problem(order, periodic=(1, 1, 1))
+    cfg["B_OVER_A"], cfg["EVALUATE_SPONGE"], cfg["BC_SPONGE_WIDTH"] = 0.0, 0, [0] * 6
+    with dg().Solver(cfg) as s:
+        rho, vel = acoustic_state(s.dims, order)
+        rho *= size * 1e3
+        for a in range(3):
+            vel[a] = 3.3e-4 * (a + 1)
+        check(cfg, dg().line_operators(order), s, rho, vel, (1, 2, 3))
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4, 5, 6, 7])
+@pytest.mark.parametrize("size", [1e-4, 1e-8, 1e-12, 1e-18])
+def test_mass_of_small_velocities_in_a_large_density(order, size):
+    """The reverse: a uniform density, whose momentum flux has no jumps, and a
+    velocity field far below a sound wave's."""
+    cfg = problem(order, periodic=(1, 1, 1), diffusion=False)
+    cfg["B_OVER_A"], cfg["EVALUATE_SPONGE"], cfg["BC_SPONGE_WIDTH"] = 0.0, 0, [0] * 6
+    with dg().Solver(cfg) as s:
+        rho, vel = acoustic_state(s.dims, order)
+        rho[:] = 0.22
+        vel *= size * 330.0
+        check(cfg, dg().line_operators(order), s, rho, vel, (0,))
