@@ -161,7 +161,7 @@ cudaError_t launch(const dg_params& p, const double* D, const double* L0, const 
     const int grid = (md.n_elem + dg::epb_of(K) - 1) / dg::epb_of(K);
     const int fix_grid = (md.n_elem + dg::fix_epb(K) - 1) / dg::fix_epb(K);
     if (p.eval_diff) {
-        if (fix_grad) dg::ldg_gradient_fix_kernel<K><<<fix_grid, dg::fix_threads(K), 0, st>>>(io, mf, G, FG);
+        if (fix_grad) dg::fix_gradient<K>(FG)<<<fix_grid, dg::fix_threads(K), 0, st>>>(io, mf, G, FG);
         else dg::ldg_gradient_kernel<double, K><<<grid, block, 0, st>>>(io, md, Gd);
         if (fix)
             dg::stage_fix_kernel<K, true, 0, false>

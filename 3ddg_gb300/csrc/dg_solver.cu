@@ -169,8 +169,9 @@ void launch_grad(Solver& s, const StageIO<T>& io, const MeshDev<T>& md)
             incr_gradient_kernel<K, false, size_t><<<grid, incr_threads(K), 0, s.stream>>>(io, md,
                                                                                           host_const<T, K>(s, 3));
     } else if (s.fix_ok[3]) {
-        launch_pdl(ldg_gradient_fix_kernel<K>, (md.n_elem + fix_epb(K) - 1) / fix_epb(K), fix_threads(K), s.stream, io,
-                   md, host_const<T, K>(s, 3), fix_set<K>(s).grad);
+        const FixOps<K, 1>& F = fix_set<K>(s).grad;
+        launch_pdl(fix_gradient<K>(F), (md.n_elem + fix_epb(K) - 1) / fix_epb(K), fix_threads(K), s.stream, io, md,
+                   host_const<T, K>(s, 3), F);
     } else {
         ldg_gradient_kernel<T, K><<<(md.n_elem + epb_of(K) - 1) / epb_of(K), dim3(npt_of(K), epb_of(K)), 0, s.stream>>>(
             io, md, const_ptr<T, K>(s, 3));

@@ -151,7 +151,8 @@ __device__ __noinline__ void grad_line_fp64(const OpConst<double, K>& C, FixGrad
     }
 }
 
-template <int K>
+// REST: the operator's RP and RQ apply (K = 2, 3, 5; always at the other orders).
+template <int K, bool REST>
 __global__ void __launch_bounds__(fix_threads(K))
 ldg_gradient_fix_kernel(StageIO<double> io, MeshDev<double> m, const __grid_constant__ OpConst<double, K> C,
                         const __grid_constant__ FixOps<K, 1> F)
@@ -204,8 +205,8 @@ ldg_gradient_fix_kernel(StageIO<double> io, MeshDev<double> m, const __grid_cons
         const int eo = E + F.line.e_out[0];
         double* out = &S.g[L.a][L.sb0];
         const FixVal X0 = fix_from(ro[r][0], E) + x[0], XN = fix_from(ro[r][1], E) + x[K - 1];
-        fix_line<K, 1>(F.line, 0, x, X0, XN, X0, XN,
-                       [&](int i, long long o) { out[i * L.sst] = fix_to_fp64(o, eo); });
+        fix_line<K, 1, REST>(F.line, 0, x, X0, XN, X0, XN,
+                             [&](int i, long long o) { out[i * L.sst] = fix_to_fp64(o, eo); });
     }
     __syncthreads();
     if (!act) return;
@@ -510,6 +511,13 @@ inline bool make_grad_fix(const OpConst<double, K>& C, FixOps<K, 1>& F)
     std::memset(&F, 0, sizeof F);
     const FixFlux f[1] = {{1.0, 0.0, 0}};
     return fix_axes<K>(C, false, F.ws, F.cube) && fix_axis<K, 1>(C.rows[0], -1, f, F.line);
+}
+
+// The gradient kernel of operator F.
+template <int K>
+inline auto fix_gradient(const FixOps<K, 1>& F)
+{
+    return fix_rest(K) || F.line.rest ? ldg_gradient_fix_kernel<K, true> : ldg_gradient_fix_kernel<K, fix_rest(K)>;
 }
 
 }  // namespace dg

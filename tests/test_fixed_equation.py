@@ -130,3 +130,49 @@ def test_unit_is_the_equations_own(K, two, shim):
         u = unit(v, w, vo, wo, jump, pm, e_out)
         err = np.abs(out.astype(q) - want)
         assert np.all(err <= 131 * u + np.abs(want) * q(2.0 ** -53)), (trial, err / u)
+
+
+@pytest.mark.parametrize("K", range(2, 9))
+@pytest.mark.parametrize("off", [1e-14, 5e-13])
+def test_operator_is_the_given_one(K, off, shim):
+    """Rows and lift columns whose mirror symmetry is broken by more than
+    rounding and less than 1e-12."""
+    rng = np.random.default_rng(1000 * K)
+    for trial in range(200):
+        rows = mirrored(K, rows_of(K, 0.01))
+        top = [np.max(np.abs(rows[:, :K])), np.max(np.abs(rows[:, K:]))]
+        for j in range(K + 2):
+            rows[:, j] += off * top[j >= K] * rng.uniform(-0.5, 0.5, K)
+        x, y, pm = 0.005, 0.004, 0
+        v, w, vo, wo = draw(rng, K, 1.0, int(rng.choice([0, 8])), bool(trial % 2))
+        jump = rng.standard_normal(2)
+        rc, out, e_out = evaluate(shim, K, rows, 0, x, y, pm, v, w, vo, wo, jump)
+        assert rc == 1
+        want = exact(K, rows, x, y, v, w, vo, wo, jump)
+        u = unit(v, w, vo, wo, jump, pm, e_out)
+        err = np.abs(out.astype(q) - want)
+        assert np.all(err <= 133 * u + np.abs(want) * q(2.0 ** -53)), (trial, err / u)
+
+
+@pytest.mark.parametrize("K", range(2, 9))
+@pytest.mark.parametrize("lumped", [False, True])
+def test_library_operators_within_solver_rounding(K, lumped, shim):
+    """The library's D and lift columns as they are: applied as given, or (K =
+    2, 3, 5) with rows that differ from them by no more than 2^-48 of the
+    largest entry, the rounding of the solve that produced them."""
+    rng = np.random.default_rng(K)
+    ops = dg().line_operators(K - 1, lumped=lumped)
+    rows = np.ascontiguousarray(np.column_stack([ops["deriv"] * 0.01, ops["lift0"], ops["liftN"]]))
+    noise = 2.0 ** -48 if K in (2, 3, 5) else 0.0
+    x, y, pm = 0.005, 0.004, 0
+    for _ in range(200):
+        v, w, vo, wo = draw(rng, K, 1.0, 0, True)
+        jump = rng.standard_normal(2)
+        rc, out, e_out = evaluate(shim, K, rows, 0, x, y, pm, v, w, vo, wo, jump)
+        assert rc == 1
+        want = exact(K, rows, x, y, v, w, vo, wo, jump)
+        f = [x * (vo[0] + wo[0] + v[0] + w[0]) + y * jump[0], -x * (vo[1] + wo[1] + v[-1] + w[-1]) + y * jump[1]]
+        slack = noise * (np.max(np.abs(rows[:, :K])) * np.sum(np.abs(v + w)) +
+                         np.max(np.abs(rows[:, K:])) * np.sum(np.abs(f)))
+        err = np.abs(out.astype(q) - want)
+        assert np.all(err <= 133 * unit(v, w, vo, wo, jump, pm, e_out) + slack + np.abs(want) * q(2.0 ** -53))

@@ -145,3 +145,80 @@ def test_mass_of_small_velocities_in_a_large_density(order, size):
         rho[:] = 0.22
         vel *= size * 330.0
         check(cfg, dg().line_operators(order), s, rho, vel, (0,))
+
+
+# ------------------------------------------------- operators from matrix files
+def operator_files(folder, order, off):
+    """Matrix and coefficient files whose S of ``order`` has one entry scaled by
+    1 + off."""
+    import refinputs
+    refinputs.write_coeff_files(str(folder))
+    path = os.path.join(str(folder), "matrices.txt")
+    with open(path, "w") as f:
+        for N in range(1, refinputs.KMAX):
+            M, S = (np.array(m, dtype=np.float64) for m in refinputs.unit_matrices(N, False))
+            if N == order:
+                S[0, 1] *= 1.0 + off
+            f.write("Order=%d\n" % N)
+            for r in np.concatenate([M, S]):
+                f.write(" ".join(refinputs.hexd(v) for v in r) + "\n")
+    return path, os.path.join(str(folder), "hardcoded_coeff.txt")
+
+
+def asymmetry(ops):
+    D = ops["deriv"]
+    return float(np.max(np.abs(D + D[::-1, ::-1])) / np.max(np.abs(D)))
+
+
+def noalloc_rhs(cfg, ops, s, ne):
+    """dg_eval_rhs_noalloc of a Solver's state with the caller's M and S."""
+    import torch
+    m = dg()
+    K = cfg["ORDER"] + 1
+    base, NP, n_elem = s.device_state()
+    index = np.arange(n_elem).reshape(ne)
+    nbr = np.empty(tuple(ne) + (6,), dtype=np.int32)
+    for a in range(3):
+        for side in (0, 1):
+            n = np.roll(index, -1 if side else 1, a).copy()
+            edge = [slice(None)] * 3
+            edge[a] = ne[a] - 1 if side else 0
+            if not cfg["BC_IS_PERIODIC"][a]:
+                n[tuple(edge)] = -1
+            nbr[..., 2 * a + side] = n
+    _, sig = s.grid()
+    d_nbr = torch.from_numpy(nbr.reshape(-1, 6)).cuda()
+    d_sig = torch.from_numpy(sig[::K, ::K, ::K].reshape(-1).copy()).cuda()
+    d_rhs = torch.full((4 * n_elem * NP,), float("nan"), dtype=torch.float64, device="cuda")
+    mass, stiff = (np.ascontiguousarray(ops[k]) for k in ("mass", "stiff"))
+    s.synchronize()
+    torch.cuda.synchronize()
+    rc = m.lib().dg_eval_rhs_noalloc(C.byref(s.params), mass.ctypes.data, stiff.ctypes.data, base[0],
+                                     d_nbr.data_ptr(), d_sig.data_ptr(), d_rhs.data_ptr(), n_elem, None)
+    assert rc == 0, m.lib().dg_last_error().decode()
+    torch.cuda.synchronize()
+    X, Y, Z = ne
+    g = d_rhs.cpu().numpy().reshape(4, X, Y, Z, NP)[..., :K ** 3].reshape(4, X, Y, Z, K, K, K)
+    return g.transpose(0, 1, 4, 2, 5, 3, 6).reshape(4, X * K, Y * K, Z * K)
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4, 5, 6, 7])
+@pytest.mark.parametrize("diffusion", [True, False])
+def test_operator_slightly_off_mirror_symmetry(order, diffusion, tmp_path):
+    """An operator off by more than rounding and less than the 1e-12 that the
+    fixed-point kernels take is applied as given, by the handle and by
+    dg_eval_rhs_noalloc."""
+    mf, cf = operator_files(tmp_path, order, 4e-13)
+    ops = dg().line_operators(order, matrix_file=mf, coeff_file=cf)
+    assert 2e-14 < asymmetry(ops) <= 1e-12
+    ne = (3, 2, 4)
+    cfg = problem(order, ne, diffusion=diffusion)
+    cfg["B_OVER_A"] = 0.0
+    with dg().Solver(cfg, mf, cf) as s:
+        rho, vel = acoustic_state(s.dims, order)
+        check(cfg, ops, s, rho, vel)
+        s.set_state(rho, vel)
+        got = noalloc_rhs(cfg, ops, s, ne)
+        want, size = Reference(cfg, ops).rhs(rho, vel, s.grid()[1])
+    for f in range(4):
+        assert float(np.max(np.abs(got[f].astype(q) - want[f]))) <= EPS * size[f]
