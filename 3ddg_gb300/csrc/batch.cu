@@ -656,7 +656,14 @@ int Batch::step(int nsteps)
             launches += step_kernels;
         } else {
             int rc = launch_step();
-            if (rc) return rc;
+            if (rc) {
+                // the launches before the failed one take tiles from the
+                // counters, which the step's last launch would have cleared:
+                // the next step uploads its tiles anew, which clears them
+                for (cudaStream_t b : branch) cudaStreamSynchronize(b);
+                tiles_dirty = true;
+                return rc;
+            }
         }
     }
     return DG_OK;
