@@ -466,7 +466,10 @@ __device__ __forceinline__ typename Pair<T>::type face_term(const OpConst<T, K>&
 // of evaluating every interior face node's neighbour flux a second time
 // (its own element evaluates it for its line sums).
 //
-template <typename T, int K, bool DIFF, int FLUX>
+// PACK: the stage's output is also written in host order to io.pack (the
+// last stage of a step whose result is downloaded: a launch of its own for
+// that took 20 to 30 us on 2.1 M nodes).
+template <typename T, int K, bool DIFF, int FLUX, bool PACK = false>
 __global__ void __launch_bounds__(npt_of(K) * epb_of(K))
 stage_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__ Cp, int do_adv, int do_sponge)
 {
@@ -607,6 +610,11 @@ stage_kernel(StageIO<T> io, MeshDev<T> m, const OpConst<T, K>* __restrict__ Cp, 
 #pragma unroll
         for (int a = 0; a < 3; a++)
             io.flux_out[(size_t)(1 + a) * io.fs + off] = mass_flux(vo[1 + a], vo[0], C.r0, C.linear_mass);
+    }
+    if constexpr (PACK) {
+        const size_t gi = grid_index(io.pack_map, e, n);
+#pragma unroll
+        for (int f = 0; f < 4; f++) io.pack[(size_t)f * io.pack_gsize + gi] = (double)vo[f];
     }
 }
 

@@ -191,14 +191,13 @@ void launch_plain_mode(const Solver& s, int slot, const StageIO<double>& io, con
                    s.stream, io, md, host_const<double, K>(s, slot), fix_set<K>(s).stage[slot], s.p.eval_advect,
                    s.p.eval_sponge);
     else
-        stage_kernel<double, K, DIFF, FLUX>
+        stage_kernel<double, K, DIFF, FLUX, PACK>
             <<<(md.n_elem + epb_of(K) - 1) / epb_of(K), dim3(npt_of(K), epb_of(K)), 0, s.stream>>>(
                 io, md, const_ptr<double, K>(s, slot), s.p.eval_advect, s.p.eval_sponge);
 }
 
 // The host-order pack rides only on the flux-reading mode (the steady state
-// of stepping with advection) of the fixed-point kernel; io.pack is set only
-// when that runs.
+// of stepping with advection); io.pack is set only when that mode runs.
 template <int K, bool DIFF>
 void launch_plain(const Solver& s, int slot, const StageIO<double>& io, const MeshDev<double>& md)
 {
@@ -397,7 +396,7 @@ int Solver::rk_stage_fp64(int s_idx, double dt, double* rhs_only)
         io.flux_in = flux_valid ? d_flux[flux_cur] : nullptr;
         io.flux_out = d_flux[1 - flux_cur];
     }
-    if (s_idx == 2 && !rhs_only && stage3_pack && io.flux_in && io.flux_out && fix_ok[s_idx]) {
+    if (s_idx == 2 && !rhs_only && stage3_pack && io.flux_in && io.flux_out) {
         io.pack = stage3_pack;
         io.pack_map = grid_map(mesh);
         io.pack_gsize = gsize();

@@ -222,3 +222,52 @@ def test_operator_slightly_off_mirror_symmetry(order, diffusion, tmp_path):
         want, size = Reference(cfg, ops).rhs(rho, vel, s.grid()[1])
     for f in range(4):
         assert float(np.max(np.abs(got[f].astype(q) - want[f]))) <= EPS * size[f]
+
+
+# 9 elements: the last block of the FP64 kernels (4 or 2 elements at orders 1 to 3) is partly filled
+@pytest.mark.parametrize("order", [1, 2, 3, 4, 5, 6, 7])
+@pytest.mark.parametrize("diffusion", [True, False])
+def test_operator_without_mirror_symmetry(order, diffusion, tmp_path):
+    """The FP64 kernels of dg_kernels.cuh, by the handle and by
+    dg_eval_rhs_noalloc (which copies the operators into its scratch and clears
+    its boundary flags for them)."""
+    mf, cf = operator_files(tmp_path, order, 1e-6)
+    ops = dg().line_operators(order, matrix_file=mf, coeff_file=cf)
+    assert asymmetry(ops) > 1e-7
+    ne = (1, 3, 3)
+    cfg = problem(order, ne, diffusion=diffusion)
+    with dg().Solver(cfg, mf, cf) as s:
+        rho, vel = acoustic_state(s.dims, order)
+        check(cfg, ops, s, rho, vel)
+        s.set_state(rho, vel)
+        got = noalloc_rhs(cfg, ops, s, ne)
+        want, size = Reference(cfg, ops).rhs(rho, vel, s.grid()[1])
+    for f in range(4):
+        assert float(np.max(np.abs(got[f].astype(q) - want[f]))) <= EPS * size[f]
+
+
+@pytest.mark.parametrize("order", [1, 2, 4, 7])
+@pytest.mark.parametrize("off", [0.0, 4e-13, 1e-6])
+def test_step_and_download_of_any_operator(order, off, tmp_path):
+    """step_state_async against step and state, bit for bit; once the fluxes of
+    the state are there, the last stage writes the host order itself (no launch
+    beyond the step's)."""
+    import torch
+    mf, cf = operator_files(tmp_path, order, off)
+    cfg = problem(order, (2, 3, 3))
+    with dg().Solver(cfg, mf, cf) as a, dg().Solver(cfg, mf, cf) as b:
+        rho, vel = acoustic_state(a.dims, order)
+        for s in (a, b):
+            s.set_state(rho, vel)
+            s.step(cfg["DT"], 1)
+        pin = lambda n: torch.empty(n, dtype=torch.float64, pin_memory=True).numpy()  # noqa: E731
+        out = pin(tuple(a.dims)), pin((3,) + tuple(a.dims))
+        before = a.launches
+        a.step(cfg["DT"], 1)
+        per_step = a.launches - before
+        before = b.launches
+        b.step_state_async(cfg["DT"], *out)
+        assert b.launches - before == per_step
+        b.synchronize()
+        r, v = a.state()
+        assert np.any(r) and np.array_equal(out[0], r) and np.array_equal(out[1], v)
