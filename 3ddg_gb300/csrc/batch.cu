@@ -549,15 +549,17 @@ int Batch::launch_step()
     const int nb = G > 1 ? std::min(G, (int)kBranches) : 0;
     if (nb) DGB_CUDA(cudaEventRecord(fork_ev, stream));
     for (int b = 0; b < nb; b++) DGB_CUDA(cudaStreamWaitEvent(branch[b], fork_ev, 0));
-    // Dependent launches only while the step's tiles all fit on the device at once:
-    // blocks that wait for their predecessor hold slots that the other branches
-    // could use.  8 problems of 4..8 elements per axis (933 tiles) 45.7 us per
-    // step without, 43.1 with; one of 6^3 (54) 24.3, 19.6; a served mix of
-    // 1300 to 2800 tiles 33.8 ms of device time without, 35.6 with (and its
-    // graph, whose edges then change with the tile counts, is instantiated anew).
+    // Dependent launches only for small steps: blocks that wait for their
+    // predecessor hold slots that the other branches could use.  The line is
+    // where the two cross, about 8 tiles per SM (us per step, waiting / dependent:
+    // 216 tiles 22.6 / 18.5, 384 26.7 / 24.5, 530 34.5 / 30.7, 777 36.8 / 30.9,
+    // 864 39.0 / 38.8, 1270 44.9 / 45.0, 2204 75.3 / 77.1, 3410 170.5 / 174.0);
+    // a served mix of 1300 to 2800 tiles took 33.8 ms of device time without, 35.6
+    // with (its graph, whose edges then change with the tile counts, is
+    // instantiated anew).
     int tiles_all = 0;
     for (const Group& grp : groups) tiles_all += grp.end - grp.begin;
-    const bool small = tiles_all <= num_sms * BATCH_GRAD_BLOCKS;
+    const bool small = tiles_all <= 8 * num_sms;
     for (int g = 0; g < G; g++) {
         const Group& grp = groups[g];
         const int K = grp.K;

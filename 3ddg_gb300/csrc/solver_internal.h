@@ -83,13 +83,22 @@ struct Solver {
 
     bool fp64() const { return p.precision == DG_PRECISION_FP64; }
     size_t gsize() const { return (size_t)mesh.n_elem * mesh.K * mesh.K * mesh.K; }
-    // FP32 launches of up to about 20 us start under the one before
-    // (launch_pdl): 8^3 elements at N = 3, 656 -> 422 us per 120 launches.  Above,
-    // the dependent form's plain loads and early wait cost more than the gap
-    // (64^3 at N = 4: 17.4 -> 19.4 ms per 48 launches; 13,800 elements at N = 3,
-    // 0.88 M nodes: 1.558 -> 1.570 ms per 120).  The FP64 kernels are always
-    // launched so: 8^3 at N = 3, 797 -> 553 us per 120; 64^3 at N = 4, 15.9 ->
-    // 15.3 ms per 18.
+    // FP32 launches of problems up to 0.8 M nodes start under the one before
+    // (launch_pdl).  The form's plain loads and early wait cost less than the
+    // gap where a problem runs alone, up to 1.7 M nodes, and where three run side
+    // by side on streams of their own, which fill each other's gaps, up to about
+    // 0.8 M, but for N = 4 and 6.  us per step, waiting / dependent:
+    //            alone                                  one of three
+    //   nodes    0.2 M    0.8 M    1.7 M      3 M       0.2 M    0.8 M    1.7 M
+    //   N = 1    41 / 26  86 / 71  171 / 155  284 / 264  19 / 17  68 / 67  153 / 150
+    //   N = 2    38 / 26  82 / 70  166 / 150  266 / 249  18 / 15  66 / 66  141 / 140
+    //   N = 3    32 / 23  67 / 53  127 / 115  209 / 196  16 / 13  48 / 49  109 / 110
+    //   N = 4    33 / 22  70 / 63  127 / 126  216 / 222  16 / 14  54 / 61  110 / 121
+    //   N = 5    40 / 26  70 / 58  148 / 136  255 / 244  18 / 16  54 / 55  134 / 135
+    //   N = 6    33 / 26  70 / 61  142 / 142  265 / 279  16 / 15  55 / 61  128 / 144
+    //   N = 7    41 / 26  81 / 71  154 / 142  265 / 255  17 / 14  70 / 71  143 / 146
+    // The FP64 kernels are always launched so: 8^3 at N = 3, 797 / 553 us per 120
+    // launches; 64^3 at N = 4, 15.9 / 15.3 ms per 18.
     bool short_launches() const { return gsize() <= 800000; }
     size_t device_bytes() const;
     void* state_ptr() const;

@@ -3,8 +3,9 @@ batch: states of 2^32 values) take, against their 32-bit forms bit for bit.
 
 The kernels take the distance of two elements in memory as an argument: a few
 elements that lie far enough apart reach the offsets of a large problem, with
-all fields interleaved in the room between them.  The shim instantiates both
-forms of each kernel from its header."""
+all fields interleaved in the room between them.  The shim instantiates the
+forms of each kernel from its header; the single-problem kernels also as a
+dependent launch."""
 import ctypes as C
 import importlib
 import os
@@ -25,7 +26,7 @@ using namespace dg;
 
 extern "C" int narrow_rules(unsigned long long fs) { return incr_narrow(fs) | batch_narrow(fs) << 1; }
 
-template <int K, typename Off>
+template <int K, bool PDL, typename Off>
 static void single(float* b, long long fs, int np, int n, const int* nbr, const float* sigma, const int* bnd_src,
                    const float* bnd_ap, const double* D, const double* L0, const double* LN)
 {
@@ -54,9 +55,13 @@ static void single(float* b, long long fs, int np, int n, const int* nbr, const 
     m.n_elem = n;
     m.src_p = 0.3f;
     const int grid = (n + incr_epb(K) - 1) / incr_epb(K), threads = incr_threads(K);
-    incr_gradient_kernel<K, false, Off><<<grid, threads>>>(io, m, G);
-    if constexpr (incr_epb(K) > 1) incr_packed_stage_kernel<K, true, false, Off><<<grid, threads>>>(io, m, S, 1, 1);
-    else incr_stage_kernel<K, true, false, Off><<<grid, threads>>>(io, m, S, 1, 1);
+    if (PDL) launch_pdl(incr_gradient_kernel<K, PDL, Off>, grid, threads, 0, io, m, G);
+    else incr_gradient_kernel<K, PDL, Off><<<grid, threads>>>(io, m, G);
+    void (*stage)(StageIO<float>, MeshDev<float>, const OpConst<float, K>, int, int);
+    if constexpr (incr_epb(K) > 1) stage = incr_packed_stage_kernel<K, true, PDL, Off>;
+    else stage = incr_stage_kernel<K, true, PDL, Off>;
+    if (PDL) launch_pdl(stage, grid, threads, 0, io, m, S, 1, 1);
+    else stage<<<grid, threads>>>(io, m, S, 1, 1);
 }
 
 template <int K, typename Off>
@@ -122,15 +127,16 @@ extern "C" int run(int form, int K, int wide, float* b, long long fs, int np, in
 {
 #define SINGLE(k)                                                                                          \
     if (form == 0 && K == k) {                                                                            \
-        if (wide) single<k, size_t>(b, fs, np, n, nbr, sigma, bnd_src, bnd_ap, D, L0, LN);               \
-        else single<k, unsigned>(b, fs, np, n, nbr, sigma, bnd_src, bnd_ap, D, L0, LN);                  \
+        if (wide == 2) single<k, true, unsigned>(b, fs, np, n, nbr, sigma, bnd_src, bnd_ap, D, L0, LN);  \
+        else if (wide) single<k, false, size_t>(b, fs, np, n, nbr, sigma, bnd_src, bnd_ap, D, L0, LN);   \
+        else single<k, false, unsigned>(b, fs, np, n, nbr, sigma, bnd_src, bnd_ap, D, L0, LN);           \
     }
 #define BATCH(k)                                                                                           \
     if (form == 1 && K == k) {                                                                            \
         if (wide) batch<k, size_t>(b, fs, np, n, nbr, sigma, (BatchProblem*)dP, (BatchTile*)dT, counters, D, L0, LN); \
         else batch<k, unsigned>(b, fs, np, n, nbr, sigma, (BatchProblem*)dP, (BatchTile*)dT, counters, D, L0, LN);    \
     }
-    SINGLE(2) SINGLE(4) SINGLE(5) SINGLE(8) BATCH(3) BATCH(5) BATCH(6)
+    SINGLE(2) SINGLE(3) SINGLE(4) SINGLE(5) SINGLE(6) SINGLE(7) SINGLE(8) BATCH(3) BATCH(5) BATCH(6)
     const cudaError_t e = cudaGetLastError();
     return (int)(e == cudaSuccess ? cudaDeviceSynchronize() : e);
 }
@@ -163,10 +169,23 @@ def test_rules(shim):
 @pytest.mark.parametrize("form,K,far", [(0, 2, 2 ** 27), (0, 4, 2 ** 27), (0, 5, 2 ** 27), (0, 8, 2 ** 27),
                                         (1, 3, 2 ** 29), (1, 5, 2 ** 29), (1, 6, 2 ** 29)])
 def test_far_elements_bitwise_as_near_ones(form, K, far, shim):
+    near = 23 * 1024
+    n = 9
+    assert K ** 3 <= 1024 and far >= near and (n - 1) * far * 4 >= 2 ** 32 and (form == 0 or (n - 1) * far >= 2 ** 32)
+    compare(form, K, ((0, near), (1, far)), shim)
+
+
+@pytest.mark.parametrize("K", range(2, 9))
+def test_dependent_launches_bitwise_as_waiting_ones(K, shim):
+    compare(0, K, ((0, 23 * 1024), (2, 23 * 1024)), shim)
+
+
+def compare(form, K, forms, shim):
+    """The outputs of the given (form, distance) pairs are the same bits."""
     import torch
     n, fs, n_fields = 9, 1024, 23
     near = n_fields * fs
-    assert K ** 3 <= fs and far >= near and (n - 1) * far * 4 >= 2 ** 32 and (form == 0 or (n - 1) * far >= 2 ** 32)
+    far = max(d for _, d in forms)
     if torch.cuda.mem_get_info()[0] < (n * far * 4 + (4 << 30)):
         pytest.skip("not enough free device memory")
     rng = np.random.default_rng(10 * K + form)
@@ -183,7 +202,7 @@ def test_far_elements_bitwise_as_near_ones(form, K, far, shim):
     ops = dg().line_operators(K - 1)
     host = [np.ascontiguousarray(ops[k]) for k in ("deriv", "lift0", "liftN")]
     out = []
-    for wide, np_slots in ((0, near), (1, far)):
+    for wide, np_slots in forms:
         buf = torch.empty(n * np_slots, dtype=torch.float32, device="cuda")
         view = buf.view(n, np_slots)[:, :near].view(n, n_fields, fs)[:, :, :K ** 3]
         view.copy_(values)
