@@ -87,9 +87,10 @@ double stage_flops(const Solver& s, bool has_old)
     return f * (double)s.gsize();
 }
 
-// Per-launch operators live in a small device buffer (one slot each for the
-// three RK stages, the LDG gradient and a bare right-hand side), rebuilt
-// only when dt changes.
+// Per-launch operators (one slot each for the three RK stages, the LDG gradient
+// and a bare right-hand side), rebuilt only when dt changes.  They are kernel
+// parameters; the FP64 kernels for operators without a fixed-point form alone
+// read them from a small device buffer.
 template <typename T, int K>
 constexpr size_t const_slot()
 {
@@ -128,13 +129,13 @@ int upload_consts_k(Solver& s, double dt)
             s.fix_ok[i] = i == 3 ? make_grad_fix<K>(C, F.grad) : make_stage_fix<K>(C, F.stage[i]);
         }
     }
-    if (!s.d_const) {
-        cudaError_t e = cudaMalloc(&s.d_const, 5 * slot);
+    if (sizeof(T) == 8 && std::count(s.fix_ok, s.fix_ok + 5, true) < 5) {
+        cudaError_t e = s.d_const ? cudaSuccess : cudaMalloc(&s.d_const, 5 * slot);
         if (e != cudaSuccess) return fail(DG_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+        // stream-ordered after every launch that used the previous operators
+        e = cudaMemcpyAsync(s.d_const, h.data(), 5 * slot, cudaMemcpyHostToDevice, s.stream);
+        if (e != cudaSuccess) return fail(DG_ERR_CUDA, std::string("cudaMemcpyAsync: ") + cudaGetErrorString(e));
     }
-    // stream-ordered after every launch that used the previous operators
-    cudaError_t e = cudaMemcpyAsync(s.d_const, h.data(), 5 * slot, cudaMemcpyHostToDevice, s.stream);
-    if (e != cudaSuccess) return fail(DG_ERR_CUDA, std::string("cudaMemcpyAsync: ") + cudaGetErrorString(e));
     s.h_const = std::move(h);
     s.const_dt = dt;
     return DG_OK;
@@ -386,7 +387,7 @@ int Solver::rk_stage_fp64(int s_idx, double dt, double* rhs_only)
     }
     md.ic_live = (s_idx == 0 && ic_live) ? 1 : 0;
     md.src_p = burst_pressure(p, tst[s_idx]);
-    if (!d_const || (!rhs_only && dt != const_dt)) {
+    if (h_const.empty() || (!rhs_only && dt != const_dt)) {
         int rc = upload_consts<double>(*this, dt);
         if (rc) return rc;
     }
@@ -447,7 +448,7 @@ int Solver::rk_stage_fp32(int s_idx, double dt, float* rhs_only)
     }
     md.ic_live = (s_idx == 0 && ic_live) ? 1 : 0;
     md.src_p = (float)burst_pressure(p, tst[s_idx]);
-    if (!d_const || (!rhs_only && dt != const_dt)) {
+    if (h_const.empty() || (!rhs_only && dt != const_dt)) {
         int rc = upload_consts<float>(*this, dt);
         if (rc) return rc;
     }

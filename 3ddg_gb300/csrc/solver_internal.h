@@ -39,10 +39,10 @@ struct Solver {
     void* d_bnd_ic = nullptr;
     void* d_bnd_ap = nullptr;
     int* d_bnd_src = nullptr;
-    void* d_const = nullptr;  // per-launch operators: 3 RK stages, LDG gradient, bare RHS
+    void* d_const = nullptr;  // FP64: h_const on the device, once an operator has no fixed-point form
     bool fix_ok[5] = {};        // FP64: the operator has a fixed-point form
     std::vector<char> h_fix;    // FP64: those forms (FixSet of dg_solver.cu)
-    std::vector<char> h_const;  // host copy of d_const (for by-value kernel parameters)
+    std::vector<char> h_const;  // per-launch operators: 3 RK stages, LDG gradient, bare RHS
     double* d_elem_b = nullptr;  // FP64: cb - ca sigma per element for the 3 RK stages
     // FP64 with advection: volume fluxes (f_mom, f_mass x, y, z) of the next
     // stage's input in d_flux[flux_cur], written by the stage that produced

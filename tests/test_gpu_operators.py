@@ -271,3 +271,26 @@ def test_step_and_download_of_any_operator(order, off, tmp_path):
         b.synchronize()
         r, v = a.state()
         assert np.any(r) and np.array_equal(out[0], r) and np.array_equal(out[1], v)
+
+
+@pytest.mark.parametrize("precision,off", [(64, 0.0), (64, 1e-6), (32, 0.0)])
+def test_operators_follow_dt(precision, off, tmp_path):
+    """Steps of changing dt, the right-hand side before the first of them and
+    between them, against the oracle with the same operator."""
+    import pyoracle
+    import refinputs
+    order = 3
+    mf, cf = operator_files(tmp_path, order, off)
+    cfg = problem(order, (3, 2, 4))
+    cfg["PRECISION"] = precision
+    o = pyoracle.Oracle(dict(cfg, PRECISION=64), *refinputs.read_matrices(mf, order), refinputs.read_zeros(cf, order))
+    tol = 1e-10 if precision == 64 else 1e-5
+    with dg().Solver(cfg, mf, cf) as s:
+        for k, f in enumerate((1.0, 0.5, 0.5, 0.75)):
+            if k != 1:
+                (r, v), (ro, vo) = s.rhs(), o.rhs()
+                assert max_rel(r, ro) <= tol and max_rel(v, vo) <= tol
+            s.step(f * cfg["DT"], 2)
+            o.run(f * cfg["DT"], 2)
+        (r, v), (ro, vo) = s.state(), o.state()
+    assert max_rel(r, ro) <= tol and max_rel(v, vo) <= tol
