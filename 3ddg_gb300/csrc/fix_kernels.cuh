@@ -228,29 +228,16 @@ struct FixSmem {
     double q[3][fix_slots(K)];
 };
 
-// One equation of a line in FP64, for values fixed point cannot hold (and lines
-// of zeros), with axis 0's operator like the fixed-point form: v (+ w) at the
-// line's nodes, g its lift-scaled face fluxes.
+// One equation of a line in FP64, for values fixed point cannot hold, with axis
+// 0's operator like the fixed-point form: v (+ w) at the line's nodes, g its
+// lift-scaled face fluxes.
 template <int K>
 __device__ __noinline__ void stage_line_fp64(const OpConst<double, K>& C, const double* pv, const double* pw, int sst,
                                              double g0, double gN, double* out)
 {
     double v[K];
-    long long any = fix_bits(g0) | fix_bits(gN);
 #pragma unroll
-    for (int j = 0; j < K; j++) {
-        v[j] = pv[j * sst];
-        any |= fix_bits(v[j]);
-        if (pw) {
-            any |= fix_bits(pw[j * sst]);
-            v[j] += pw[j * sst];
-        }
-    }
-    if (any << 1 == 0) {  // +-0 everywhere
-#pragma unroll 1
-        for (int j = 0; j < K; j++) out[j * sst] = 0.0;
-        return;
-    }
+    for (int j = 0; j < K; j++) v[j] = pw ? pv[j * sst] + pw[j * sst] : pv[j * sst];
 #pragma unroll 1
     for (int i = 0; i < K; i++) {
         const double* row = C.rows[0][i];

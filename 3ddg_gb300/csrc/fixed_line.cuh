@@ -273,7 +273,8 @@ __host__ __device__ __forceinline__ int fix_abs_hi_at(const double* p)
 // equation's fluxes are, of which it sees no more than the jumps, formed in
 // FP64.  (One exponent for both lost the smaller: at u = 3.3e-4 m/s-scale mass
 // fluxes and drho = 1e-8 the momentum sums were off by 5e-8 of their largest.)
-// False, and nothing written, when fixed point cannot hold the values.
+// False, and nothing written, when fixed point cannot hold the values (zeros it
+// can).
 template <int K, bool TWO>
 __host__ __device__ __forceinline__ bool fix_equation(const FixLine<K, 2>& L, int eq, int py, const double* v,
                                                       const double* w, int st, const double (&vo)[2],
@@ -286,8 +287,19 @@ __host__ __device__ __forceinline__ bool fix_equation(const FixLine<K, 2>& L, in
         t = fix_max(t, fix_abs_hi_at(v + j * st));
         if (TWO) t = fix_max(t, fix_abs_hi_at(w + j * st));
     }
-    const int E = fix_max(t >> 20, (fix_max(fix_abs_hi(y0), fix_abs_hi(yN)) >> 20) - py);
-    if (E < kFixMinExp || E > kFixMaxExp) return false;
+    const int ty = fix_max(fix_abs_hi(y0), fix_abs_hi(yN)), E = fix_max(t >> 20, (ty >> 20) - py);
+    if (E < kFixMinExp || E > kFixMaxExp) {
+        // zeros are all there is ahead of a wave: no arithmetic for them
+        if ((t | ty) != 0) return false;
+        int low = (int)(fix_bits(vo[0]) | fix_bits(vo[1]) | fix_bits(y0) | fix_bits(yN));
+        if (TWO) low |= (int)(fix_bits(wo[0]) | fix_bits(wo[1]));
+#pragma unroll
+        for (int j = 0; j < K; j++) low |= (int)(fix_bits(v[j * st]) | (TWO ? fix_bits(w[j * st]) : 0));
+        if (low) return false;
+#pragma unroll
+        for (int j = 0; j < K; j++) out[j * st] = 0.0;
+        return true;
+    }
     FixVal x[K], X0 = fix_from(vo[0], E), XN = fix_from(vo[1], E);
 #pragma unroll
     for (int j = 0; j < K; j++) x[j] = fix_from(v[j * st], E);

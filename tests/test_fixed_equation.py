@@ -176,3 +176,28 @@ def test_library_operators_within_solver_rounding(K, lumped, shim):
                          np.max(np.abs(rows[:, K:])) * np.sum(np.abs(f)))
         err = np.abs(out.astype(q) - want)
         assert np.all(err <= 133 * unit(v, w, vo, wo, jump, pm, e_out) + slack + np.abs(want) * q(2.0 ** -53))
+
+
+@pytest.mark.parametrize("K", range(2, 9))
+@pytest.mark.parametrize("two", [False, True])
+def test_zeros_and_what_is_left_to_fp64(K, two, shim):
+    """Lines of +-0 give +0; one denormal, huge or non-finite value anywhere
+    leaves the line to the caller, untouched."""
+    rows = rows_of(K, 0.01)
+
+    def line(fill):
+        v, vo, jump = np.full(K, fill), np.full(2, fill), np.full(2, fill)
+        return v, np.full(K, fill) if two else None, vo, np.full(2, fill) if two else None, jump
+
+    for fill in (0.0, -0.0):
+        rc, out, _ = evaluate(shim, K, rows, 0, 0.005, 0.004, 0, *line(fill))
+        assert rc == 1 and not out.any() and not np.signbit(out).any()
+    for bad in (5e-324, -1e-310, 2.0 ** -900, 2.0 ** 900, np.inf, np.nan):
+        for which in range(5):
+            for fill in (0.0, 1.0) if abs(bad) > 1 or bad != bad else (0.0,):
+                a = line(fill)
+                if a[which] is None:
+                    continue
+                a[which][-1] = bad
+                rc, _, _ = evaluate(shim, K, rows, 0, 0.005, 0.004, 0, *a)
+                assert rc == 0, (bad, which, fill)
