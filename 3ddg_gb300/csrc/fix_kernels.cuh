@@ -1,8 +1,9 @@
 // FP64 kernels of one RK stage with the line operators in block fixed point
 // (fixed_line.cuh): the LDG gradient and the stage update.  Fields, fluxes and
-// the RK combination are FP64 (16 FP64 operations per node and stage); what is
-// linear with constant coefficients (line sums, face terms, lifts) is integer
-// work of the line owners, which runs beside the FP64 pipe.
+// the RK combination are FP64 (16 FP64 operations per node and stage), as are the
+// jumps across the faces (4 per line); what is linear with constant coefficients
+// (line sums, face terms, lifts) is integer work of the line owners, which runs
+// beside the FP64 pipe.
 //
 // Mapping: a CTA takes fix_epb(K) whole elements.  In the node phases thread t
 // has node t of the CTA's nodes, in the line phase line t of its lines (3 K^2
@@ -293,18 +294,22 @@ __device__ __forceinline__ void stage_fix_line(const OpConst<double, K>& C, cons
 // What bounds these kernels and what they measured (ms per launch at 32.8 M
 // nodes, even-odd or per-node FP64 line sums -> fixed point):
 //   K          2           3           4           5           6           7           8
-//   stage      8.99->1.40  4.49->1.41  3.85->1.18  3.85->1.32  4.28->1.41  4.69->1.66  5.67->1.51
+//   stage      8.99->1.74  4.49->1.54  3.85->1.31  3.85->1.44  4.28->1.54  4.69->1.77  5.67->1.66
 //   gradient   1.54->0.55  1.10->0.41  1.11->0.41  1.11->0.38  1.40->0.49  1.60->0.51  1.69->0.52
-// (with one exponent for both equations of a line; fix_equation has the cost of
-// one each).  At K = 5 a stage launch kept the FP64 pipe 69 % busy (16 operations
-// per node), the integer pipe 53 %, the issue slots 62 % and HBM at 71 % of a copy:
-// no unit is the bound by itself, the barriers between the node and line phases
-// are (26 % of the warps' time), so resident warps count most.  Registers per
-// thread of the stage kernel and elements per CTA were chosen by that (us per
-// launch on 8 M nodes: K = 5 at 40 / 48 / 56 / 80 registers 335 / 329 / 358 /
-// 537; K = 8 at 32 / 40 / 48 380 / 404 / 494; K = 4 at 1 / 2 / 4 / 6 elements
-// 383 / 296 / 311 / 349; with an exponent per equation K = 2 at 48 / 56 / 64
-// registers 448 / 432 / 459, the other orders as before).  Converting results on the FP64 pipe (fix_to_fp64)
+// At K = 5 a stage launch keeps the FP64 pipe 73 % busy, the integer pipe 54 %,
+// the issue slots 61 % and HBM at 66 % of a copy: no unit is the bound by itself,
+// the barriers between the node and line phases are (a quarter of the warps'
+// time), so resident warps count most.  Registers per thread of the stage kernel
+// and elements per CTA were chosen by that.  us per launch on 8 M nodes at 32 / 40 /
+// 48 / 56 / 64 registers:
+//   K = 2  686 / 527 / 448 / 432 / 459    K = 6  536 / 537 / 389 / 377 / 411
+//   K = 3  572 / 384 / 387 / 417 / 417    K = 7  572 / 422 / 410 / 410 / 535
+//   K = 4  414 / 373 / 329 / 334 / 334    K = 8  408 / 439 / 512 / 512 / 512
+//   K = 5  497 / 366 / 355 / 390 / 389
+// and, before an exponent per equation, K = 4 at 1 / 2 / 4 / 6 elements 383 / 296 /
+// 311 / 349.  At the registers chosen the kernels that read fluxes spill 0 to 28
+// bytes per thread up to K = 7 and 210 to 300 at K = 8, where more registers cost
+// more in resident warps.  Converting results on the FP64 pipe (fix_to_fp64)
 // instead saves integer work where that pipe is the scarcer one: 346 for 329 us.
 __host__ __device__ constexpr int fix_regs(int K) { return K == 8 ? 32 : K == 6 || K == 2 ? 56 : 48; }
 __host__ __device__ constexpr int fix_min_blocks(int K) { return 65536 / (fix_regs(K) * fix_threads(K)); }
@@ -481,8 +486,9 @@ inline bool make_stage_fix(const OpConst<double, K>& C, FixOps<K, 2>& F)
             if (!(std::fabs(C.cM[0][s][i] - m[s][i]) <= tm) || !(std::fabs(C.cA[0][s][i] - r[s][i]) <= tr)) return false;
         if (!(std::fabs(C.cQ[0][s] - (s ? -h : h)) <= 1e-14 * std::fabs(h))) return false;
     }
-    // momentum fluxes enter times 2^pm ~ rho0 / c, the ratio of the mass to the
-    // momentum flux of a sound wave
+    // jumps of the momentum flux enter the mass equation times 2^pm ~ rho0 / c (of
+    // the mass flux the momentum equation times 2^-pm), so that their coefficients
+    // are of the size of the others
     const double k = h != 0.0 ? g / h : 1.0;
     if (!(k > 0x1p-40 && k < 0x1p40)) return false;
     F.pm = (int)std::lround(std::log2(k));

@@ -14,14 +14,26 @@
 // that the 3 bits that sums of a line's values grow by need no carry, and a
 // product is three mad.wide.s32 (the fourth, low x low, is dropped).
 //
-// Error: truncating a value loses less than 2^-56 of the line's largest, a
-// product drops less than half of that unit, a sum is floored once at an
-// eighth of it: about 2^-56 of (largest value x row sum), where a chain of
-// K + 4 FP64 operations rounds to 2^-53 of its partial sums each time.
+// Error: the largest of a line's values is 2^55 to 2^56 units, truncating a value
+// loses less than a unit, a product drops its low x low part, a sum is floored
+// once at an eighth of a unit.  In all at most 131 eighths, scaled by the row sum
+// (test_fixed_line.py), that is 66 x 2^-55 of (largest value x row sum); a chain
+// of K + 4 FP64 operations rounds to 2^-53 of its partial sums each time.
+// Measured on lines of resolved sound waves, see fix_equation: 4 to 40 times
+// below FP64 sums.
+//
+// The bound is one of the line, not of the row: a value more than 8 times below
+// the largest keeps fewer than 53 bits, and a row that gives the largest little
+// weight is the less precise for it.  Random values, each 1/8 of its neighbour
+// on the line, rms error at K = 4 / 5 / 8 (FP64 sums in brackets): of the line's
+// largest result 2.5e-16 / 2.5e-16 / 2.6e-16 (2.7e-16 / 2.0e-16 / 3.8e-16), of
+// each row's own absolute sum 2.4e-16 / 5.0e-16 / 7.4e-16 (1.5e-16 / 1.9e-16 /
+// 1.7e-16), and with lumped mass, whose inner rows do not see the neighbours,
+// 5.9e-15 / 8.3e-15 / 1.9e-14 (1.1e-16 / 4.8e-15 / 1.1e-16).
 //
 // What fixed point cannot hold (an infinity or NaN on the line, a largest
 // value outside 2^-823 .. 2^877) is left to an FP64 evaluation of that line by
-// the caller; so is a line of zeros and denormals.
+// the caller; so is a line of denormals.
 #pragma once
 
 #include <cmath>
@@ -196,7 +208,7 @@ template <int K, int NEQ>
 struct FixOps {
     FixLine<K, NEQ> line;
     double ws[3];  // w_0 / w_a
-    int pm;        // momentum fluxes enter scaled by 2^pm
+    int pm;        // jumps enter the other equation scaled by 2^pm (make_stage_fix)
     int cube;      // ws is 1
 };
 
@@ -271,8 +283,16 @@ __host__ __device__ __forceinline__ int fix_abs_hi_at(const double* p)
 // out may be the same memory.  The exponent is that of the largest of these
 // values alone: an equation's sums keep their bits however large the other
 // equation's fluxes are, of which it sees no more than the jumps, formed in
-// FP64.  (One exponent for both lost the smaller: at u = 3.3e-4 m/s-scale mass
-// fluxes and drho = 1e-8 the momentum sums were off by 5e-8 of their largest.)
+// FP64.  One exponent for both equations needs no FP64 subtractions and fewer
+// conversions (us per stage launch on 8 M nodes, K = 2 .. 8: 359 / 361 / 300 / 337 /
+// 352 / 389 / 384, this form 439 / 389 / 330 / 362 / 380 / 410 / 419; at rest 363 /
+// 346 / 269 / 297 / 281 / 301 / 287 and 375 / 372 / 313 / 323 / 310 / 310 / 320), but
+// loses the smaller flux: 5e-8 of the momentum sums at 1e-8 of a sound wave's
+// density.  Lines of resolved sound waves (3 to 12 elements long), rms error of
+// a sum in units of its own absolute sum, K = 2 .. 8: one exponent 3.7e-16 /
+// 3.4e-16 / 5.6e-16 / 8.1e-16 / 6.0e-16 / 1.3e-15 / 2.8e-15, this form 1.2e-17 /
+// 7.5e-17 / 1.9e-17 / 2.4e-17 / 2.1e-17 / 4.2e-17 / 4.1e-17, FP64 sums 5.2e-16 /
+// 4.8e-16 / 3.0e-16 / 2.6e-16 / 2.6e-16 / 2.3e-16 / 4.0e-16.
 // False, and nothing written, when fixed point cannot hold the values (zeros it
 // can).
 template <int K, bool TWO>

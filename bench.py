@@ -424,7 +424,7 @@ def run_ours(a, dist: Dist):
                           "frac": ((st_f / st_n) / (st_ms / st_n / 1e3) / 1e12) / FP64_PEAK_TFLOPS if st_n else None,
                           "note": "flops counted by the direct formula (K (K + 2) per line); the line sums run as "
                                   "block fixed point on the integer pipes, so that this exceeds the FP64 pipe's "
-                                  "1.19 TFLOP/s; 12 to 16 operations per node and stage are left on that pipe"},
+                                  "1.19 TFLOP/s; 12 to 16 operations per node and 4 per line are left on that pipe per stage"},
             "share_of_step": st_ms / ms if ms else None,
             "gradient_kernel": {"name": ("ldg_gradient_fix_kernel<%d>" if fp64 else "incr_gradient_kernel<%d>")
                                 % (cfg["ORDER"] + 1),

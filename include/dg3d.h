@@ -161,7 +161,10 @@ int dg_eval_rhs(dg_handle* h, double* drho, double* vel);
  * value in [-6*n_elem, -1], for a boundary face, whose exterior state is zero;
  * the table is not checked, and any other entry is undefined behaviour), d_sigma (n_elem sponge sigmas; may be NULL when
  * eval_sponge is 0) and d_rhs (output, same layout as d_state); host mass and
- * stiff are the (N+1)^2 unit-interval matrices of matrices.txt.  FP64 only,
+ * stiff are the (N+1)^2 unit-interval matrices of matrices.txt (the operator
+ * M^-1 S is applied as solved, except that at orders 1, 2 and 4 rows that
+ * mirror each other to the rounding of that solve, 2^-51 (order 1) or 2^-48 of
+ * the largest entry, are applied as exact mirror images).  FP64 only,
  * order 1..7, at most DG_NOALLOC_MAX_ELEMENTS elements and
  * DG_NOALLOC_MAX_NODES node slots (larger problems are rejected with
  * DG_ERR_INVALID).  Calls no cudaMalloc/cudaFree or other allocating routine:
